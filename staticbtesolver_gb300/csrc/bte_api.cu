@@ -25,6 +25,7 @@
 
 #include "../../include/bte_cuda.h"
 #include "bte_kernels.cuh"
+#include "bte_krylov.cuh"
 #include "bte_transport.cuh"
 #include "bte_mlp.cuh"
 #include "bte_dsa.cuh"
@@ -129,6 +130,12 @@ struct bte_ctx {
     double* h_pinned = nullptr;  // [4]
     int* h_pinned_i = nullptr;   // [4]
     std::vector<int> h_done, h_iters;
+    // k_bicg_cluster: inflow slots (0 not known), cells per CTA for this
+    // problem's batches by precision (0: FP64, 1: FP32; 0 cells: the phase
+    // kernels, -1 not decided) and the batch size it was decided for
+    int kc_slots = 0;
+    int kc_len[2] = {-1, -1};
+    int kc_systems[2] = {0, 0};
     // learned accelerator
     std::vector<double> centroid;
     bool has_mlp = false;
@@ -664,6 +671,8 @@ static bte_status setup(bte_ctx* ctx, int batch_systems) {
     ctx->h_done.resize(S);
     ctx->h_iters.resize(S);
     ctx->plan_ready = false;
+    ctx->kc_slots = 0;
+    ctx->kc_len[0] = ctx->kc_len[1] = -1;
     ctx->mixed_ready = false;
     ctx->dsa_ready = false;
     ctx->dirty = false;
@@ -1329,8 +1338,130 @@ static bool krylov_persistent() {
     return v && v[0] == 'p' && v[1] == 'e';
 }
 
+// ---------------------------------------------------------------------------
+// One cluster per system (k_bicg_cluster).
+
+template <typename Op, typename T>
+static const void* cluster_kernel(int slots) {
+    // CTAs per SM the registers are limited for: two in FP64 (as many full ones
+    // fit in shared memory), three in FP32
+    constexpr int minb = sizeof(T) == 8 ? 2 : 3;
+    if constexpr (std::is_same<Op, bte::CsrOp>::value) return (const void*)bte::k_bicg_cluster<Op, T, 0, minb>;
+    else
+        return slots == 2 ? (const void*)bte::k_bicg_cluster<Op, T, 2, minb>
+               : slots == 3 ? (const void*)bte::k_bicg_cluster<Op, T, 3, minb>
+                            : (const void*)bte::k_bicg_cluster<Op, T, 4, minb>;
+}
+
+// Launch configuration of S clusters of ctas CTAs; attr must outlive cfg.
+template <typename T>
+static cudaLaunchConfig_t cluster_config(int S, int ctas, int len, int slots, bool best, cudaStream_t st,
+                                         cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg = {};
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)ctas;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)S * (unsigned)ctas);
+    cfg.blockDim = dim3(bte::THREADS);
+    cfg.dynamicSmemBytes = bte::cluster_smem_bytes<T>(len, slots, best);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Cells per CTA for S systems of n cells, or 0: the phase kernels (more than
+// KC_CTAS CTAs' cells, or clusters that do not fit the device).  A system gets
+// the fewest CTAs its cells need: remote neighbour values and cluster barriers
+// cost more than a fuller SM (20,000 cells x 256 systems: 10 CTAs 81 ms, 12
+// 107 ms, 16 172 ms; 10,082 cells in FP32: 5 CTAs 25 ms, 6 28 ms, 8 38 ms).
+// While that leaves SMs without one it gets more, of at least kClusterSpread
+// cells (578 cells x 32 systems: 1 CTA and 4 CTAs 17 ms, the barriers then cost
+// what the FP64 pipes gain).
+constexpr int kClusterSpread = 512;
+template <typename Op, typename T>
+static int cluster_len(int device, int S, int n, int slots) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+    // (with three or four slots in FP64, two CTAs share an SM up to 1,792 cells)
+    const int cells = sizeof(T) == 8 && slots > 2 && n <= 1792 * bte::KC_CTAS ? 1792 : bte::KC_CELLS;
+    const int ctas = std::max((n + cells - 1) / cells, std::min({bte::KC_CTAS, sms / S, n / kClusterSpread}));
+    if (ctas > bte::KC_CTAS) return 0;
+    const int len = ((n + ctas - 1) / ctas + 31) & ~31;
+    const void* k = cluster_kernel<Op, T>(slots);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config<T>(S, (n + len - 1) / len, len, slots, true, nullptr, &attr);
+    int clusters = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    return len;
+}
+
+template <typename Op, typename T>
+static cudaError_t launch_cluster(const Op& op, const T* rhs, size_t Np, int S, int slots, const bte::ClusterSolve& cs,
+                                  cudaStream_t st) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg =
+        cluster_config<T>(S, (cs.n + cs.len - 1) / cs.len, cs.len, slots, cs.best != 0, st, &attr);
+    void* args[] = {(void*)&op, (void*)&rhs, (void*)&Np, (void*)&cs};
+    return cudaLaunchKernelExC(&cfg, cluster_kernel<Op, T>(slots), args);
+}
+
+// How the S systems of a plain batch ended, into the report.
+static bte_status batch_outcome(bte_ctx* ctx, int S, bte_report& rep) {
+    cudaStream_t st = ctx->stream;
+    BTE_CUDA(cudaMemcpyAsync(ctx->h_done.data(), ctx->s_done.p, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
+    BTE_CUDA(cudaMemcpyAsync(ctx->h_iters.data(), ctx->s_iters.p, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
+    BTE_CUDA(cudaStreamSynchronize(st));
+    for (int y = 0; y < S; ++y) {
+        rep.inner_iterations += ctx->h_iters[y];
+        if (ctx->h_done[y] == 3 || ctx->h_done[y] == 0) ++rep.inner_unconverged;
+    }
+    rep.inner_solves += S;
+    return BTE_OK;
+}
+
+// Cells per CTA for a batch of S systems of ctx in *len (0: the phase
+// kernels), decided once per set-up and batch size (prec: 0 FP64, 1 FP32).  The
+// profiler times the phases one by one, so a profiled solve takes the phase
+// kernels; so does BTE_KRYLOV=phase, and =persistent its own kernel.
+template <typename Op, typename T>
+static bte_status batch_len(bte_ctx* ctx, int S, int prec, int* len) {
+    *len = 0;
+    const char* v = std::getenv("BTE_KRYLOV");
+    if (ctx->profile || (v && v[0] == 'p') || ctx->n > bte::KC_CELLS * bte::KC_CTAS) return BTE_OK;
+    if (ctx->kc_slots == 0) {  // face slots: the largest inflow count
+        BTE_CUDA(ctx->m_active.alloc(sizeof(int)));
+        BTE_CUDA(cudaMemsetAsync(ctx->m_active.p, 0, sizeof(int), ctx->stream));
+        bte::k_max_inflow<<<dim3((ctx->n + 255) / 256, ctx->n_dir), 256, 0, ctx->stream>>>(
+            ctx->d_fc.as<double>(), ctx->F, ctx->n, ctx->Np, ctx->m_active.as<int>());
+        BTE_LAUNCHED();
+        BTE_CUDA(cudaMemcpyAsync(ctx->h_pinned_i, ctx->m_active.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        BTE_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->kc_slots = std::max(2, ctx->h_pinned_i[0]);
+    }
+    if (ctx->kc_slots > 4) return BTE_OK;
+    if (ctx->kc_len[prec] < 0 || ctx->kc_systems[prec] != S) {
+        ctx->kc_len[prec] = cluster_len<Op, T>(ctx->device, S, ctx->n, ctx->kc_slots);
+        ctx->kc_systems[prec] = S;
+    }
+    *len = ctx->kc_len[prec];
+    return BTE_OK;
+}
+
 static bte_status solve_batch_plain(bte_ctx* ctx, int b0, int nbb, const bte_options& o, bte_report& rep) {
+    int len = 0;
     {
+        bte_status s = batch_len<bte::FaceFluxOp, double>(ctx, nbb * ctx->n_dir, 0, &len);
+        if (s != BTE_OK) return s;
+    }
+    if (len > 0) {
+        BTE_CUDA(ctx->w_b.alloc(sizeof(double) * (size_t)ctx->nbb * ctx->n_dir * ctx->Np));
+    } else {
         const size_t bytes = sizeof(double) * (size_t)ctx->nbb * ctx->n_dir * ctx->Np;
         for (DevBuf* b : {&ctx->w_r, &ctx->w_rw, &ctx->w_p, &ctx->w_ph, &ctx->w_q, &ctx->w_z, &ctx->w_t, &ctx->w_b,
                           &ctx->w_invD, &ctx->w_xb})
@@ -1356,6 +1487,14 @@ static bte_status solve_batch_plain(bte_ctx* ctx, int b0, int nbb, const bte_opt
                    ctx->w_b.as<double>(), ctx->n));
 
     const int maxit = o.inner_maxit;
+    if (len > 0) {
+        const int cyc = std::max(1, o.plain_cycles);
+        const bte::ClusterSolve cs{ctx->s_done.as<int>(), ctx->s_iters.as<int>(), nullptr, ctx->n, len,
+                                   o.inner_tol, maxit, cyc, cyc > 1 ? maxit / 2 : 0, cyc > 1};
+        BTE_CUDA(launch_cluster(op, (const double*)ctx->w_b.as<double>(), ctx->Np, S, ctx->kc_slots, cs, st));
+        BTE_LAUNCHED();
+        return batch_outcome(ctx, S, rep);
+    }
     // The reference stops a system at maxit and keeps its last iterate
     // (cycles = 1, no best-iterate copy).  With plain_cycles = k > 1 a system
     // not converged after maxit iterations goes on up to k x maxit and keeps
@@ -1404,21 +1543,14 @@ static bte_status solve_batch_plain(bte_ctx* ctx, int b0, int nbb, const bte_opt
         if (ctx->h_pinned_i[0] == 0 || last > total) break;
         if (i > total + 1) break;
     }
-    BTE_CUDA(cudaMemcpyAsync(ctx->h_done.data(), ctx->s_done.p, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-    BTE_CUDA(cudaMemcpyAsync(ctx->h_iters.data(), ctx->s_iters.p, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
     if (ctx->profile) {
         ctx->h_active.resize(total + 2);
         BTE_CUDA(cudaMemcpyAsync(ctx->h_active.data(), ctx->s_active.p, sizeof(int) * (total + 2),
                                  cudaMemcpyDeviceToHost, st));
+        BTE_CUDA(cudaStreamSynchronize(st));
+        prof_resolve(ctx, ctx->h_active.data(), total + 2);
     }
-    BTE_CUDA(cudaStreamSynchronize(st));
-    if (ctx->profile) prof_resolve(ctx, ctx->h_active.data(), total + 2);
-    for (int y = 0; y < S; ++y) {
-        rep.inner_iterations += ctx->h_iters[y];
-        if (ctx->h_done[y] == 3 || ctx->h_done[y] == 0) ++rep.inner_unconverged;
-    }
-    rep.inner_solves += S;
-    return BTE_OK;
+    return batch_outcome(ctx, S, rep);
 }
 
 // Mixed form for one batch: x starts from the previous outer iterate; each
@@ -1462,6 +1594,11 @@ static bte_status solve_batch_mixed(bte_ctx* ctx, int b0, int nbb, const bte_opt
                            ctx->x_t.as<float>(), ctx->x_b.as<float>(), ctx->x_invD.as<float>(), ctx->Np};
     v.xb = ctx->x_xb.as<float>();
     const double w = 4.0;
+    int len = 0;
+    {
+        bte_status s = batch_len<bte::FaceFluxOp32, float>(ctx, S, 1, &len);
+        if (s != BTE_OK) return s;
+    }
     const int max_cycles = 30;
     int cycle = 0;
     for (; cycle < max_cycles; ++cycle) {
@@ -1476,6 +1613,13 @@ static bte_status solve_batch_mixed(bte_ctx* ctx, int b0, int nbb, const bte_opt
         BTE_CUDA(cudaMemcpyAsync(ctx->h_pinned_i + 1, ctx->m_active.p, sizeof(int), cudaMemcpyDeviceToHost, st));
         BTE_CUDA(cudaStreamSynchronize(st));
         if (ctx->h_pinned_i[1] == 0) break;
+        if (len > 0) {
+            BTE_CUDA(launch_cluster(op32, (const float*)ctx->x_b.as<float>(), ctx->Np, S, ctx->kc_slots,
+                                    bte::ClusterSolve{ctx->s_done.as<int>(), ctx->s_iters.as<int>(),
+                                                      ctx->m_skip.as<int>(), ctx->n, len, 1e-4, maxit, 1, 0, 1},
+                                    st));
+            BTE_LAUNCHED();
+        } else {
         BTE_CUDA(cudaMemsetAsync(ctx->s_active.p, 0, sizeof(int) * (maxit + 2), st));
         BTE_LAUNCH(KK_INIT, -1, S * N * 7 * w + geo32 / 2, 0,
                    bte::k_bicg_init<<<grid, bte::THREADS, 0, st>>>(op32, v, bs));
@@ -1509,6 +1653,7 @@ static bte_status solve_batch_mixed(bte_ctx* ctx, int b0, int nbb, const bte_opt
                                      cudaMemcpyDeviceToHost, st));
             BTE_CUDA(cudaStreamSynchronize(st));
             prof_resolve(ctx, ctx->h_active.data(), maxit + 2);
+        }
         }
         BTE_LAUNCH(KK_X, -1, S * N * (8.0 * 2 + 4.0), 0,
                    bte::k_mixed_update<<<grid, bte::THREADS, 0, st>>>(op, ctx->x_dx.as<float>(),

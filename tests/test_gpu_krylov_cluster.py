@@ -1,0 +1,90 @@
+"""The Krylov forms' BiCGSTAB with one thread-block cluster per system
+(k_bicg_cluster) against the phase kernels, which a profiled solve takes (it
+times the phases one by one).  Both run the same iteration with differently
+grouped sums and coefficients, so they agree to what the inner tolerance
+leaves: each system ends at a relative residual below inner_tol = 1e-9, and
+the error of x is at most that times the condition of the Jacobi-scaled
+operator, of the order of the upwind graph's depth (under 100 levels here):
+2 x 1e-9 x 50 = 1e-7 relative in the intensities.  Iteration counts differ by
+rounding only (5 %).  A second cluster solve gives the same bits."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# one cell more or less than a row of 256 threads, a full CTA and the largest
+# cluster; systems few enough to spread over several CTAs, and many
+CELLS = [1, 2, 33, 255, 256, 257, 2047, 2048, 2049, 4097, 20000, 32767, 32768, 32769]
+MESHES = [("square16_b8", 0), ("square10_b40", 0), ("2DM2DG", 0), ("3DM2DG", 0), ("cube4_b2", 0), ("cube7_b1", 4),
+          ("cube14_b1", 2)]
+
+
+def _both(sbte, problem, close=1e-7, tol_=1e-5, **kw):
+    out = []
+    for profile in (True, False, False):
+        ctx = sbte.Context(0)
+        ctx.set_arrays(problem) if isinstance(problem, dict) else ctx.load(problem)
+        st, rep = ctx.solve(profile=profile, tol=tol_, **kw)
+        out.append((st, ctx.energy(), ctx.temperature(), rep.as_dict()))
+        if profile:
+            assert ctx.kernel_stats()["bicg_spmv1"]["launches"] > 0
+        ctx.close()
+    (s0, e0, _, r0), (s1, e1, T1, r1), (s2, e2, T2, _) = out
+    assert s0 == s1 == s2
+    assert np.array_equal(e1, e2) and np.array_equal(T1, T2)
+    assert np.linalg.norm(e1 - e0) <= close * np.linalg.norm(e0)
+    for k in ("n_iter", "inner_solves") + (("inner_unconverged",) if np.isfinite(close) else ()):
+        assert r0[k] == r1[k], k
+    assert abs(r0["inner_iterations"] - r1["inner_iterations"]) <= 0.05 * r0["inner_iterations"] + 2
+    return r0, r1
+
+
+@pytest.mark.parametrize("form", ["PLAIN", "MIXED"])
+@pytest.mark.parametrize("name,max_iter", MESHES)
+def test_cluster_equals_phase_kernels(sbte, get_case, tmp_path, name, max_iter, form):
+    from staticbtesolver_gb300 import synth
+
+    try:
+        c = get_case(name)
+        args, limit = c.args(), c.max_iter
+    except Exception:
+        p = synth.make_problem(name, str(tmp_path))
+        args, limit = (p.geo, p.bc_file, p.band_file, p.DM, p.num_theta, p.num_phi, p.T_ref, p.L_x, p.L_y, p.L_z), 1000
+    r0, r1 = _both(sbte, sbte.Problem(*args), max_iter=max_iter or limit, form=getattr(sbte, "FORM_" + form))
+    assert r1["kernel_launches"] < r0["kernel_launches"]  # one launch instead of five per iteration
+
+
+@pytest.fixture(scope="module")
+def wide_mesh(sbte, tmp_path_factory):
+    """33,282 triangles, to be cut to the first so many cells."""
+    from staticbtesolver_gb300 import synth
+
+    p = synth.make_problem("nondelaunay129_b1", str(tmp_path_factory.mktemp("wide")))
+    return sbte.Problem(p.geo, p.bc_file, p.band_file, p.DM, p.num_theta, p.num_phi, p.T_ref, p.L_x, p.L_y,
+                        p.L_z).arrays()
+
+
+@pytest.mark.parametrize("form", ["PLAIN", "MIXED"])
+@pytest.mark.parametrize("cells", CELLS)
+def test_cluster_cell_counts(sbte, wide_mesh, cells, form):
+    """The first `cells` triangles; a face cut open becomes part of the wall of entity 0."""
+    a = dict(wide_mesh, n_cell=cells)
+    for k in ("nbr", "area", "normal", "volume", "centroid"):
+        a[k] = a[k][:cells]
+    a["nbr"] = np.where(a["nbr"] >= cells, -1, a["nbr"])
+    r0, r1 = _both(sbte, a, max_iter=2, tol_=0.0, form=getattr(sbte, "FORM_" + form))
+    if cells <= 32768:
+        assert r1["kernel_launches"] < r0["kernel_launches"]
+
+
+@pytest.mark.parametrize("kw", [dict(inner_maxit=1), dict(inner_maxit=7), dict(plain_cycles=3, inner_maxit=11),
+                                dict(inner_tol=1e-14), dict(batch_systems=96)])
+def test_cluster_limits_and_batches(sbte, get_case, kw):
+    """Iteration limits (with and without the best iterate), a tight tolerance,
+    band batches.  Iterates cut off before they converge follow rounding (the
+    first right-hand sides live on wall cells, and r_hat . r falls to rounding
+    level once r has left them), so there only the counts are compared, the
+    number of systems that just meet the tolerance by then excepted."""
+    cut = kw.get("inner_maxit", 1000) < 100
+    _both(sbte, sbte.Problem(*get_case("square16_b8").args()), max_iter=4, tol_=0.0,
+          close=np.inf if cut else 1e-7, **kw)
