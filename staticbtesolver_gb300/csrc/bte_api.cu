@@ -1428,12 +1428,15 @@ static bte_status batch_outcome(bte_ctx* ctx, int S, bte_report& rep) {
 // Cells per CTA for a batch of S systems of ctx in *len (0: the phase
 // kernels), decided once per set-up and batch size (prec: 0 FP64, 1 FP32).  The
 // profiler times the phases one by one, so a profiled solve takes the phase
-// kernels; so does BTE_KRYLOV=phase, and =persistent its own kernel.
+// kernels; so does BTE_KRYLOV=phase, and =persistent its own kernel.  1D keeps
+// the phase kernels and their rounding: there r_hat . r falls to rounding level
+// within a few steps, some systems of every run end at the iteration limit, and
+// which ones do depends on the last bit of every sum.
 template <typename Op, typename T>
 static bte_status batch_len(bte_ctx* ctx, int S, int prec, int* len) {
     *len = 0;
     const char* v = std::getenv("BTE_KRYLOV");
-    if (ctx->profile || (v && v[0] == 'p') || ctx->n > bte::KC_CELLS * bte::KC_CTAS) return BTE_OK;
+    if (ctx->profile || (v && v[0] == 'p') || ctx->dim == 1 || ctx->n > bte::KC_CELLS * bte::KC_CTAS) return BTE_OK;
     if (ctx->kc_slots == 0) {  // face slots: the largest inflow count
         BTE_CUDA(ctx->m_active.alloc(sizeof(int)));
         BTE_CUDA(cudaMemsetAsync(ctx->m_active.p, 0, sizeof(int), ctx->stream));
