@@ -114,20 +114,22 @@ typedef struct bte_report {
                                   whole iteration, replayed as a CUDA graph) */
     double ms_reduce;          /* temperature / margin reductions and the accelerator */
     long long kernel_launches; /* kernels this library launched during the solve */
-    int sweep_group;           /* sweep form: bands per block and threads per block */
-    int sweep_threads;         /* chosen by timing candidate shapes on a plan's first sweep */
+    int sweep_group;           /* sweep form: bands per block and threads per block, chosen by a model */
+    int sweep_threads;         /* of the launch (stream kernel) or by timing candidates on a plan's first sweep */
     int accel_steps;           /* outer-iteration extrapolations (accel 1, 2) or mixes (3) applied */
     int accel_reverts;         /* extrapolations undone (state restored) */
     int sweep_ring;            /* sweep form: solved positions kept in shared memory per band */
     int sweep_margin;          /* sweep form, acyclic plan: 1 the sweep sums the margin, 0 the reduction
-                                  does (timed against each other with the launch shape) */
+                                  does (always with the stream kernel; else timed with the launch shape) */
     int dsa_solves;            /* low-order corrections applied (dsa) */
     long long dsa_iterations;  /* conjugate-gradient iterations summed over them */
     double ms_dsa;             /* device time of the corrections (included in ms_reduce and ms_total) */
-    int sweep_kernel;          /* sweep form: the kernel the autotuner chose -- 0 level-synchronous (k_sweep),
-                                  1 staged (levels copied to shared memory ahead by bulk copies, right-hand
-                                  side from a level-ordered pre-pass), 2 level-synchronous over levels
-                                  split into slices of one position per thread */
+    int sweep_kernel;          /* sweep form: the kernel that ran -- 3 stream (k_sweep_stream: everything but
+                                  the solution brought to shared memory ahead), taken whenever the plan
+                                  suits it; else the autotuner's choice: 0 level-synchronous (k_sweep), 1
+                                  staged (levels copied to shared memory ahead by bulk copies), 2
+                                  level-synchronous over levels split into slices of one position per
+                                  thread */
     double ms_host_setup;      /* host wall time of this call's set-up after new inputs (uploads, geometry) */
     double ms_host_plan;       /* ... of building the sweep plan (level order, layout) after new geometry */
     double ms_host_order;      /*     of which the level order (host threads over directions) */
@@ -261,14 +263,14 @@ bte_status bte_mlp_train(const float* X, const float* Y, int M, int steps, int b
 bte_status bte_get_kernel_stats(bte_ctx* ctx, bte_kernel_stat* stats, int cap, int* n);
 
 /* The sweep autotuner's table from the first sweep of the current plan (empty
- * when the choice came from the per-process cache): candidate k ran with
+ * when the stream kernel ran, whose shape is not timed, or the choice came from
+ * the per-process cache): candidate k ran with
  * group[k] bands and threads[k] threads per block and ring[k] positions per
  * band, with kernel[k] (0 level-synchronous, 1 staged, 2 split levels, as
  * bte_report.sweep_kernel), in ms[k] milliseconds.  Entries are written up
  * to cap (arrays may be NULL when cap is 0); *n = candidates timed.  The
- * environment variable BTE_SWEEP_KERNEL=level|staged|split restricts the
- * candidates to one kernel (the temperatures are the same to the bit either
- * way). */
+ * environment variable BTE_SWEEP_KERNEL=level|staged|split|stream restricts the
+ * choice to one kernel (the temperatures are the same to the bit either way). */
 bte_status bte_get_sweep_tuning(bte_ctx* ctx, int* group, int* threads, int* ring, int* kernel, float* ms, int cap,
                                 int* n);
 

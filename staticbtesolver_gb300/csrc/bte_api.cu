@@ -27,6 +27,7 @@
 #include "bte_kernels.cuh"
 #include "bte_krylov.cuh"
 #include "bte_transport.cuh"
+#include "bte_stream.cuh"
 #include "bte_mlp.cuh"
 #include "bte_dsa.cuh"
 #include "dsa_setup.h"
@@ -81,8 +82,11 @@ struct SweepShape {
     bool margin = false;  // acyclic plans: the sweep sums the margin partials (else k_reduce does)
     bool staged = false;  // k_sweep_staged (levels staged by bulk copies, right-hand side formed a stage ahead)
     bool split = false;   // k_sweep over the levels split into slices of cap positions (one per thread)
-    int cap = 0;          // staged, split: positions per stage
-    int kind() const { return staged ? 1 : split ? 2 : 0; }
+    bool stream = false;  // k_sweep_stream
+    int cap = 0;          // staged, split, stream: positions per stage
+    int WC = 0, H = 0, NCH = 0, A = 0;  // stream: StreamShape
+    bte::StreamShape stream_shape() const { return {G, WC, H, W, A, NCH, cap}; }
+    int kind() const { return stream ? 3 : staged ? 1 : split ? 2 : 0; }
 };
 
 // Stage bounds of the staged sweep for one stage width: per direction, its
@@ -156,8 +160,19 @@ struct bte_ctx {
     // staged sweep: plan records, level-ordered right-hand side of a batch,
     // error flag of its bounded waits, stage lists by width; row length n2
     DevBuf p_rec, d_sweep_err;
+    bool rec_ready = false;
+    bool level_ready = false;  // the level-ordered arrays above (the level, split and staged kernels')
+    // stream kernel: padded positions (row starts of the levels, cell -> position
+    // and back), k/D and V Omega/D by band and position, stage lists by cap;
+    // records, annex entries and their counts for one (W, cap, NCH, A)
+    bool stream_ready = false;
+    DevBuf st_lrow, st_pos, st_cell, st_voi, st_kinv, st_rec, st_far, st_nfar;
+    std::map<int, std::unique_ptr<StageList>> stream_lists;
+    std::vector<int> plan_lrow;  // start rows of the levels, as plan_lvl
+    int stream_nq = 0, stream_width = 0;  // chunks of the longest direction; positions of the widest level
+    int stream_key[4] = {0, 0, 0, 0};
     // level-order work: inflow masks, order, positions, level starts, in-degrees, counts
-    DevBuf lo_mask, lo_perm, lo_pos, lo_lvl, lo_indeg, lo_small, lo_down;
+    DevBuf lo_mask, lo_perm, lo_pos, lo_lvl, lo_indeg, lo_small, lo_down, lo_lag;
     int plan_host_dirs = 0;  // directions the last plan ordered on the host
     std::vector<int> plan_lvl, plan_lvl_off;  // host copies of the level starts
     std::map<int, std::unique_ptr<StageList>> stage_lists;
@@ -1221,26 +1236,16 @@ static bte_status build_sweep_plan(bte_ctx* ctx) {
     }
     h_off[ND] = (int)h_lvl.size();
     tm.lap("order arrays");
-    // cell -> position from the order on the device; the lagged-edge flags
-    // only when some direction has a cycle (none on planar meshes)
-    DevBuf d_lag;
-    BTE_CUDA(ctx->lo_pos.alloc(sizeof(int) * (size_t)ND * n));
-    bte::k_inverse_perm<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(ctx->lo_perm.as<int>(), n, ctx->lo_pos.as<int>());
-    BTE_LAUNCHED();
+    // the lagged-edge flags only when some direction has a cycle (none on planar meshes)
     if (lagged_dirs > 0) {
         std::vector<int> h_lag((size_t)ND * F * n, 0);
         for (int d = 0; d < ND; ++d)
             if (!lag[d].empty()) std::copy(lag[d].begin(), lag[d].end(), h_lag.begin() + (size_t)d * F * n);
-        BTE_CUDA(upload(d_lag, h_lag, st));
+        BTE_CUDA(upload(ctx->lo_lag, h_lag, st));
+        BTE_CUDA(cudaStreamSynchronize(st));  // h_lag goes out of scope
     }
     BTE_CUDA(upload(ctx->p_lvl, h_lvl, st));
     BTE_CUDA(upload(ctx->p_lvl_off, h_off, st));
-    BTE_CUDA(ctx->p_cell.alloc(sizeof(int) * ND * n));
-    BTE_CUDA(ctx->p_dg.alloc(sizeof(double) * ND * n));
-    BTE_CUDA(ctx->p_vo.alloc(sizeof(double) * ND * n));
-    BTE_CUDA(ctx->p_nb.alloc(sizeof(int) * ND * F * n));
-    BTE_CUDA(ctx->p_fc.alloc(sizeof(double) * ND * F * n));
-    BTE_CUDA(ctx->p_bidx.alloc(sizeof(int) * ND * n));
     BTE_CUDA(ctx->d_bsum.alloc(sizeof(double) * (size_t)ctx->nbb * ND * std::max(ctx->nbcell, 1)));
     BTE_CUDA(ctx->p_binvd.alloc(sizeof(double) * (size_t)ctx->n_band * ND * std::max(ctx->nbcell, 1)));
     if (ctx->nbcell > 0) {
@@ -1249,59 +1254,32 @@ static bte_status build_sweep_plan(bte_ctx* ctx) {
             ctx->d_vo.as<double>(), ctx->n_band, ND, Np, ctx->p_binvd.as<double>());
         BTE_LAUNCHED();
     }
-    bte::k_sweep_layout<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(
-        ctx->lo_perm.as<int>(), ctx->lo_pos.as<int>(), lagged_dirs > 0 ? d_lag.as<int>() : nullptr, ctx->d_dg.as<double>(), ctx->d_vo.as<double>(), ctx->d_fc.as<double>(),
-        ctx->d_nbr.as<int>(), ctx->d_bidx.as<int>(), F, n, Np, ND, ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(),
-        ctx->p_dg.as<double>(), ctx->p_vo.as<double>(), ctx->p_nb.as<int>(), ctx->p_fc.as<double>());
-    BTE_LAUNCHED();
-    ctx->n2 = (n + 1) & ~1;
-    tm.lap("layout");
-    BTE_CUDA(ctx->p_voi.alloc(sizeof(double) * ctx->n_band * ND * (size_t)ctx->n2));
-    BTE_CUDA(ctx->p_kinv.alloc(sizeof(double) * ctx->n_band * ND * (size_t)ctx->n2));
-    {
-        bte::SweepPlan sp{ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_dg.as<double>(), ctx->p_vo.as<double>(), ctx->p_nb.as<int>(),
-                          ctx->p_fc.as<double>(), ctx->p_lvl.as<int>(), ctx->p_lvl_off.as<int>(), n, F, ctx->n2};
-        bte::k_sweep_invd<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(sp, ctx->d_kb.as<double>(), ctx->n_band, ND,
-                                                                     ctx->p_voi.as<double>(),
-                                                                     ctx->p_kinv.as<double>());
-        BTE_LAUNCHED();
+    BTE_CUDA(ctx->d_sweep_err.alloc(sizeof(int)));
+    BTE_CUDA(cudaMemsetAsync(ctx->d_sweep_err.p, 0, sizeof(int), st));
+    ctx->plan_lvl.swap(h_lvl);  // (outlive the uploads)
+    ctx->plan_lvl_off.swap(h_off);
+    ctx->stage_lists.clear();
+    ctx->stream_lists.clear();
+    ctx->rec_ready = ctx->level_ready = ctx->stream_ready = false;
+    ctx->stream_key[0] = 0;
+    // rows of 32 positions, each level from a row of its own
+    ctx->plan_lrow.assign(ctx->plan_lvl.size(), 0);
+    int most_rows = 0, widest = 0;
+    for (int d = 0; d < ND; ++d) {
+        const int l0 = ctx->plan_lvl_off[d], l1 = ctx->plan_lvl_off[d + 1] - 1;
+        int r = 0;
+        for (int l = l0; l < l1; ++l) {
+            ctx->plan_lrow[l] = r;
+            const int w = (ctx->plan_lvl[l + 1] - ctx->plan_lvl[l] + 31) / 32;
+            widest = std::max(widest, w);
+            r += w;
+        }
+        ctx->plan_lrow[l1] = r;
+        most_rows = std::max(most_rows, r);
     }
-    tm.lap("per-system diagonal");
-    // staged sweep: one record per (direction, position), the batch's
-    // level-ordered right-hand side, the error flag of its bounded waits
-    {
-        const int fmx = sweep_slots(ctx);
-        const int rb = fmx == 2 ? bte::SweepRecLayout<2>::bytes
-                                : fmx == 3 ? bte::SweepRecLayout<3>::bytes : bte::SweepRecLayout<4>::bytes;
-        BTE_CUDA(ctx->p_rec.alloc((size_t)rb * ND * n));
-        const dim3 g((n + 255) / 256, ND);
-        if (fmx == 2)
-            bte::k_sweep_records<2><<<g, 256, 0, st>>>(ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_nb.as<int>(),
-                                                       ctx->p_fc.as<double>(), n, F, ND,
-                                                       ctx->p_rec.as<unsigned char>());
-        else if (fmx == 3)
-            bte::k_sweep_records<3><<<g, 256, 0, st>>>(ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_nb.as<int>(),
-                                                       ctx->p_fc.as<double>(), n, F, ND,
-                                                       ctx->p_rec.as<unsigned char>());
-        else
-            bte::k_sweep_records<4><<<g, 256, 0, st>>>(ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_nb.as<int>(),
-                                                       ctx->p_fc.as<double>(), n, F, ND,
-                                                       ctx->p_rec.as<unsigned char>());
-        BTE_LAUNCHED();
-        BTE_CUDA(ctx->d_sweep_err.alloc(sizeof(int)));
-        BTE_CUDA(cudaMemsetAsync(ctx->d_sweep_err.p, 0, sizeof(int), st));
-        int smem_max = 0;
-        BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-        BTE_CUDA(cudaFuncSetAttribute(bte::k_sweep_staged<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
-        BTE_CUDA(cudaFuncSetAttribute(bte::k_sweep_staged<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
-        BTE_CUDA(cudaFuncSetAttribute(bte::k_sweep_staged<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
-        ctx->plan_lvl = h_lvl;
-        ctx->plan_lvl_off = h_off;
-        ctx->stage_lists.clear();
-    }
-    tm.lap("records");
-    BTE_CUDA(cudaStreamSynchronize(st));  // d_perm / d_lag go out of scope
-    tm.lap("sync");
+    ctx->stream_nq = (32 * most_rows + bte::SCH - 1) / bte::SCH;
+    ctx->stream_width = 32 * widest;
+    tm.lap("boundary rows, stages");
     ctx->sweep_tuned = false;
     ctx->sweep_tune_cand.clear();
     ctx->sweep_tune_ms.clear();
@@ -1310,6 +1288,70 @@ static bte_status build_sweep_plan(bte_ctx* ctx) {
     BTE_CUDA(ctx->d_spart.alloc(sizeof(double) * ND * ctx->n_band));
     ctx->plan_levels = levels;
     ctx->plan_ready = true;
+    return BTE_OK;
+}
+
+// The level-ordered plan arrays of the level, split and staged kernels, on
+// their first use with a plan.
+static bte_status level_plan(bte_ctx* ctx) {
+    if (ctx->level_ready) return BTE_OK;
+    const int n = ctx->n, F = ctx->F, ND = ctx->n_dir;
+    const size_t Np = ctx->Np;
+    cudaStream_t st = ctx->stream;
+    BTE_CUDA(ctx->lo_pos.alloc(sizeof(int) * (size_t)ND * n));
+    bte::k_inverse_perm<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(ctx->lo_perm.as<int>(), n, ctx->lo_pos.as<int>());
+    BTE_LAUNCHED();
+    BTE_CUDA(ctx->p_cell.alloc(sizeof(int) * ND * n));
+    BTE_CUDA(ctx->p_dg.alloc(sizeof(double) * ND * n));
+    BTE_CUDA(ctx->p_vo.alloc(sizeof(double) * ND * n));
+    BTE_CUDA(ctx->p_nb.alloc(sizeof(int) * ND * F * n));
+    BTE_CUDA(ctx->p_fc.alloc(sizeof(double) * ND * F * n));
+    BTE_CUDA(ctx->p_bidx.alloc(sizeof(int) * ND * n));
+    bte::k_sweep_layout<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(
+        ctx->lo_perm.as<int>(), ctx->lo_pos.as<int>(), ctx->plan_lagged_dirs > 0 ? ctx->lo_lag.as<int>() : nullptr,
+        ctx->d_dg.as<double>(), ctx->d_vo.as<double>(), ctx->d_fc.as<double>(), ctx->d_nbr.as<int>(),
+        ctx->d_bidx.as<int>(), F, n, Np, ND, ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_dg.as<double>(),
+        ctx->p_vo.as<double>(), ctx->p_nb.as<int>(), ctx->p_fc.as<double>());
+    BTE_LAUNCHED();
+    ctx->n2 = (n + 1) & ~1;
+    BTE_CUDA(ctx->p_voi.alloc(sizeof(double) * ctx->n_band * ND * (size_t)ctx->n2));
+    BTE_CUDA(ctx->p_kinv.alloc(sizeof(double) * ctx->n_band * ND * (size_t)ctx->n2));
+    bte::SweepPlan sp{ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_dg.as<double>(), ctx->p_vo.as<double>(),
+                      ctx->p_nb.as<int>(), ctx->p_fc.as<double>(), ctx->p_lvl.as<int>(), ctx->p_lvl_off.as<int>(), n, F,
+                      ctx->n2};
+    bte::k_sweep_invd<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(sp, ctx->d_kb.as<double>(), ctx->d_Cb.as<double>(),
+                                                                 ctx->solid_angle, ctx->n_band, ND,
+                                                                 ctx->p_voi.as<double>(), ctx->p_kinv.as<double>());
+    BTE_LAUNCHED();
+    ctx->level_ready = true;
+    return BTE_OK;
+}
+
+// The padded positions and their coefficients for the stream kernel, on its
+// first use with a plan.
+static bte_status stream_plan(bte_ctx* ctx) {
+    if (ctx->stream_ready) return BTE_OK;
+    const int n = ctx->n, F = ctx->F, ND = ctx->n_dir;
+    const size_t npad = (size_t)ctx->stream_nq * bte::SCH;
+    cudaStream_t st = ctx->stream;
+    BTE_CUDA(upload(ctx->st_lrow, ctx->plan_lrow, st));
+    BTE_CUDA(ctx->st_pos.alloc(sizeof(int) * (size_t)ND * n));
+    BTE_CUDA(ctx->st_cell.alloc(sizeof(int) * ND * npad));
+    BTE_CUDA(cudaMemsetAsync(ctx->st_cell.p, 0xff, sizeof(int) * ND * npad, st));
+    int most = 0;
+    for (int d = 0; d < ND; ++d) most = std::max(most, ctx->plan_lvl_off[d + 1] - 1 - ctx->plan_lvl_off[d]);
+    bte::k_stream_order<<<dim3((most + 7) / 8, ND), 256, 0, st>>>(
+        ctx->lo_perm.as<int>(), ctx->lo_mask.as<uint8_t>(), ctx->p_lvl.as<int>(), ctx->p_lvl_off.as<int>(),
+        ctx->st_lrow.as<int>(), n, F, npad, ctx->st_pos.as<int>(), ctx->st_cell.as<int>());
+    BTE_LAUNCHED();
+    BTE_CUDA(ctx->st_voi.alloc(sizeof(double) * ctx->n_band * ND * npad));
+    BTE_CUDA(ctx->st_kinv.alloc(sizeof(double) * ctx->n_band * ND * npad));
+    bte::k_stream_invd<<<dim3((unsigned)((npad + 255) / 256), ND), 256, 0, st>>>(
+        ctx->st_cell.as<int>(), ctx->d_dg.as<double>(), ctx->d_vo.as<double>(), ctx->d_kb.as<double>(),
+        ctx->d_Cb.as<double>(), ctx->solid_angle, ctx->n_band, ND, ctx->Np, npad, ctx->st_voi.as<double>(),
+        ctx->st_kinv.as<double>());
+    BTE_LAUNCHED();
+    ctx->stream_ready = true;
     return BTE_OK;
 }
 
@@ -1693,7 +1735,7 @@ static int sweep_margin_restriction() {
 static int sweep_kernel_restriction() {
     const char* v = std::getenv("BTE_SWEEP_KERNEL");
     if (!v || !*v) return -1;
-    return v[0] == 'l' ? 0 : v[0] == 's' && v[1] == 't' ? 1 : v[0] == 's' && v[1] == 'p' ? 2 : -1;
+    return v[0] == 'l' ? 0 : !std::strcmp(v, "staged") ? 1 : !std::strcmp(v, "split") ? 2 : !std::strcmp(v, "stream") ? 3 : -1;
 }
 // BTE_SWEEP_SHAPE=G,T restricts the autotuner to G bands and T threads per
 // block (a test of a particular shape, e.g. stages narrower than a level);
@@ -1736,7 +1778,7 @@ static std::vector<SweepShape> sweep_candidates(const bte_ctx* ctx, int nbb, int
     std::vector<SweepShape> out;
     for (int split = 0; split < 2; ++split)
         for (const auto& c : cand) {
-            if (only_kernel == 1 || only_kernel == (split ? 0 : 2)) break;
+            if (only_kernel == 1 || only_kernel == 3 || only_kernel == (split ? 0 : 2)) break;
             if (only_shape >= 0 && only_shape != c[0] * 10000 + c[1]) continue;
             // split levels only in the 128-thread shapes of up to 4 bands (the
             // others were never faster unsplit)
@@ -1802,15 +1844,200 @@ static bte_status stage_list(bte_ctx* ctx, int cap, const StageList** out) {
     return BTE_OK;
 }
 
+// Records of k_sweep_staged (one per direction and position), on its first use
+// with a plan.
+static bte_status staged_records(bte_ctx* ctx) {
+    if (ctx->rec_ready) return BTE_OK;
+    const int n = ctx->n, F = ctx->F, ND = ctx->n_dir, fm = sweep_slots(ctx);
+    const int rb = fm == 2 ? bte::SweepRecLayout<2>::bytes
+                           : fm == 3 ? bte::SweepRecLayout<3>::bytes : bte::SweepRecLayout<4>::bytes;
+    BTE_CUDA(ctx->p_rec.alloc((size_t)rb * ND * n));
+    const dim3 g((n + 255) / 256, ND);
+    int smem_max = 0;
+    BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+#define BTE_STAGED_REC(FM)                                                                                          \
+    do {                                                                                                            \
+        bte::k_sweep_records<FM><<<g, 256, 0, ctx->stream>>>(ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(),           \
+                                                             ctx->p_nb.as<int>(), ctx->p_fc.as<double>(), n, F, ND,  \
+                                                             ctx->p_rec.as<unsigned char>());                       \
+        BTE_CUDA(cudaFuncSetAttribute(bte::k_sweep_staged<FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max)); \
+    } while (0)
+    if (fm == 2) BTE_STAGED_REC(2);
+    else if (fm == 3) BTE_STAGED_REC(3);
+    else BTE_STAGED_REC(4);
+#undef BTE_STAGED_REC
+    BTE_LAUNCHED();
+    ctx->rec_ready = true;
+    return BTE_OK;
+}
+
+template <bool BUILD>
+static void launch_stream_records(const bte_ctx* ctx, const SweepShape& sh, int* most) {
+    const bte::StreamBuild sb{ctx->st_cell.as<int>(), ctx->st_pos.as<int>(), ctx->d_bidx.as<int>(),
+                              ctx->d_nbr.as<int>(), ctx->d_fc.as<double>(),
+                              ctx->plan_lagged_dirs > 0 ? ctx->lo_lag.as<int>() : nullptr, ctx->n, ctx->F,
+                              ctx->stream_nq, ctx->Np, (size_t)ctx->stream_nq * bte::SCH};
+    const dim3 g((ctx->stream_nq + 7) / 8, ctx->n_dir);
+    const int fm = sweep_slots(ctx);
+#define BTE_STREAM_REC(FM)                                                                                      \
+    bte::k_stream_records<FM, BUILD><<<g, 256, 0, ctx->stream>>>(sb, sh.stream_shape(), sh.W - sh.cap,           \
+                                                                 ctx->st_rec.as<unsigned char>(),               \
+                                                                 ctx->st_far.as<unsigned>(), ctx->st_nfar.as<int>(), most)
+    if (fm == 2) BTE_STREAM_REC(2);
+    else if (fm == 3) BTE_STREAM_REC(3);
+    else BTE_STREAM_REC(4);
+#undef BTE_STREAM_REC
+}
+
+static size_t stream_smem(int fm, const SweepShape& sh) {
+    return fm == 2 ? bte::stream_smem_bytes<2>(sh.stream_shape())
+                   : fm == 3 ? bte::stream_smem_bytes<3>(sh.stream_shape()) : bte::stream_smem_bytes<4>(sh.stream_shape());
+}
+
+// Annex places the shape needs per chunk (sh.A), and its shared memory.
+static bte_status stream_annex(bte_ctx* ctx, SweepShape& sh) {
+    BTE_CUDA(ctx->m_active.alloc(sizeof(int)));
+    BTE_CUDA(cudaMemsetAsync(ctx->m_active.p, 0, sizeof(int), ctx->stream));
+    launch_stream_records<false>(ctx, sh, ctx->m_active.as<int>());
+    BTE_LAUNCHED();
+    BTE_CUDA(cudaMemcpyAsync(ctx->h_pinned_i + 2, ctx->m_active.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    BTE_CUDA(cudaStreamSynchronize(ctx->stream));
+    sh.A = (ctx->h_pinned_i[2] + 1) & ~1;
+    sh.smem = stream_smem(sweep_slots(ctx), sh);
+    return BTE_OK;
+}
+
+// The plan's records for shape sh, built on its first use with a plan.
+static bte_status stream_records(bte_ctx* ctx, const SweepShape& sh) {
+    if (ctx->stream_key[0] == sh.W && ctx->stream_key[1] == sh.cap && ctx->stream_key[2] == sh.NCH &&
+        ctx->stream_key[3] == sh.A)
+        return BTE_OK;
+    const int fm = sweep_slots(ctx);
+    const size_t nd = (size_t)ctx->n_dir, nq = ctx->stream_nq;
+    const size_t rb = fm == 2 ? bte::StreamRec<2>::bytes : fm == 3 ? bte::StreamRec<3>::bytes : bte::StreamRec<4>::bytes;
+    BTE_CUDA(ctx->st_rec.alloc(rb * nd * nq * bte::SCH));
+    BTE_CUDA(ctx->st_far.alloc(sizeof(unsigned) * nd * nq * fm * bte::SCH));
+    BTE_CUDA(ctx->st_nfar.alloc(sizeof(int) * nd * nq));
+    launch_stream_records<true>(ctx, sh, nullptr);
+    BTE_LAUNCHED();
+    const void* k = fm == 2 ? (const void*)bte::k_sweep_stream<2>
+                            : fm == 3 ? (const void*)bte::k_sweep_stream<3> : (const void*)bte::k_sweep_stream<4>;
+    int smem_max = 0;
+    BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    BTE_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    ctx->stream_key[0] = sh.W;
+    ctx->stream_key[1] = sh.cap;
+    ctx->stream_key[2] = sh.NCH;
+    ctx->stream_key[3] = sh.A;
+    return BTE_OK;
+}
+
+// The stream kernel's shape for batches of nbb bands into ctx->sweep_shape;
+// *found = false: the plan does not suit it (levels so narrow that padding them
+// to rows would take more than the state itself and kStreamFree bytes, or so
+// wide that no ring holds a few of them).
+//
+// A model of the launch instead of timing candidates: its constants (cycles)
+// were fitted to 250 shapes on each of 18 plans (2D 128 to 100,352 triangles, 3D
+// 3,072 to 131,712 tetrahedra, 1 to 40 bands); the shape it picks takes 1.5 %
+// longer than the fastest one on average and 8 % at most, and a plan of a new
+// mesh costs no trial sweeps (before: ~20, 100 ms on 100,352 triangles).  Per
+// stage, the slowest of
+//  * a consumer warp's rows one after the other, with a barrier;
+//  * the FP64 pipe over the systems that share an SM;
+//  * the chunks' way through copy and helpers, NCH of them in flight;
+// times the waves of blocks.
+constexpr size_t kStreamFree = (size_t)256 << 20;
+static bte_status stream_choose(bte_ctx* ctx, int nbb, bool* found) {
+    *found = false;
+    const int fm = sweep_slots(ctx), cap = ctx->stream_width;
+    const size_t npad = (size_t)ctx->stream_nq * bte::SCH;
+    if (cap <= 0 || (npad > 2 * ctx->Np && 16 * npad * ctx->n_band * ctx->n_dir > kStreamFree)) return BTE_OK;
+    static const double kRow[3] = {520, 850, 900}, kFp64[3] = {136, 171, 200};
+    constexpr double kBarrier = 100, kPipe = 11600;
+    int smem_max = 0, sms = 0, smem_sm = 0, regs_sm = 0, threads_sm = 0;
+    BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    BTE_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
+    BTE_CUDA(cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, ctx->device));
+    BTE_CUDA(cudaDeviceGetAttribute(&threads_sm, cudaDevAttrMaxThreadsPerMultiProcessor, ctx->device));
+    BTE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    long long rows = 0;
+    for (int d = 0; d < ctx->n_dir; ++d) rows += ctx->plan_lrow[ctx->plan_lvl_off[d + 1] - 1];
+    const double per = (double)rows / std::max(1ll, ctx->plan_levels);  // rows per level
+    for (int annex = cap / 16 + 8, tries = 0; tries < 4; ++tries) {
+        SweepShape best;
+        double best_cost = 1e300;
+        for (int nch = 4; nch <= 8; nch *= 2)
+            for (int G = 1; G <= std::min(nbb, 10); ++G)
+                for (int WC = 1; WC <= 6; ++WC) {
+                    SweepShape sh;
+                    sh.stream = true;
+                    sh.G = G;
+                    sh.WC = WC;
+                    sh.NCH = sh.H = nch;
+                    sh.cap = cap;
+                    sh.A = annex;
+                    // a ring of four or five of the widest levels: older values go
+                    // through the annexes (132,000 tetrahedra, levels up to 1,568:
+                    // 8,192 positions 6.3 ms, 4,096 7.1 ms)
+                    sh.W = 1024;
+                    while (sh.W < std::max(cap + (nch + 1) * bte::SCH, 9 * cap / 2)) sh.W <<= 1;
+                    sh.threads = 32 * (G * WC + nch + 1);
+                    sh.smem = stream_smem(fm, sh);
+                    if (sh.smem > (size_t)smem_max || sh.threads > bte::STHREADS ||
+                        !bte::stream_shape_ok(sh.stream_shape()))
+                        continue;
+                    const int fit = std::min({smem_sm / (int)(sh.smem + 1024), regs_sm / (80 * sh.threads),
+                                              threads_sm / sh.threads});
+                    if (fit < 1) continue;
+                    const int blocks = (nbb + G - 1) / G * ctx->n_dir;
+                    const int waves = (blocks + sms * fit - 1) / (sms * fit);
+                    const int share = std::min(fit, (blocks + sms - 1) / sms);  // blocks on the fullest SM
+                    const double cost = waves * std::max({(per / WC + 0.25) * kRow[fm - 2] + kBarrier,
+                                                          per * G * share * kFp64[fm - 2], per / 4 * kPipe / (nch - 1)});
+                    if (cost < best_cost) {
+                        best_cost = cost;
+                        best = sh;
+                    }
+                }
+        if (!(best_cost < 1e300)) return BTE_OK;
+        bte_status s = stream_plan(ctx);
+        if (s == BTE_OK) s = stream_annex(ctx, best);
+        if (s != BTE_OK) return s;
+        if (best.smem <= (size_t)smem_max) {
+            ctx->sweep_shape = best;
+            *found = true;
+            return BTE_OK;
+        }
+        annex = best.A;  // more than assumed: choose again
+    }
+    return BTE_OK;
+}
+
 // One sweep of bands b0 .. b0+nbb-1 in every direction with shape sh, for the
 // plan's face slots (2 in 1D and 2D, 3 in 3D).
 template <bool MARGIN>
 static void launch_sweep(const bte_ctx* ctx, const SweepShape& sh, int nbb, int b0, cudaStream_t st,
-                         const bte::SweepPlan& sp, const bte::SweepSrc& src, int first_sweep, double* mpart) {
+                         const bte::SweepSrc& src, int first_sweep, double* mpart) {
     const dim3 grid((nbb + sh.G - 1) / sh.G, ctx->n_dir);
     const double* voi = ctx->p_voi.as<double>();
     const double* kinv = ctx->p_kinv.as<double>();
     const int fm = sweep_slots(ctx);
+    if (sh.stream) {  // (leaves the margin to k_reduce)
+        const StageList* sl = ctx->stream_lists.find(sh.cap)->second.get();
+        const bte::StreamPlan pl{ctx->st_rec.as<unsigned char>(), ctx->st_far.as<unsigned>(), ctx->st_nfar.as<int>(),
+                                 sl->stages.as<int>(), sl->off.as<int>(), ctx->stream_nq};
+#define BTE_STREAM_FM(FM)                                                                                            \
+    bte::k_sweep_stream<FM><<<grid, sh.threads, sh.smem, st>>>(pl, sh.stream_shape(), ctx->st_kinv.as<double>(),      \
+                                                               ctx->st_voi.as<double>(), src, ctx->e_curr,           \
+                                                               first_sweep, nbb, b0, ctx->n_dir, ctx->Np,            \
+                                                               ctx->d_sweep_err.as<int>())
+        if (fm == 2) BTE_STREAM_FM(2);
+        else if (fm == 3) BTE_STREAM_FM(3);
+        else BTE_STREAM_FM(4);
+#undef BTE_STREAM_FM
+        return;
+    }
     if (sh.staged) {  // MARGIN is false here: the staged kernel leaves the margin to k_reduce
         const StageList* sl = ctx->stage_lists.find(sh.cap)->second.get();
         const bte::StagedPlan pl{ctx->p_rec.as<unsigned char>(), sl->stages.as<int>(), sl->off.as<int>(),
@@ -1825,7 +2052,9 @@ static void launch_sweep(const bte_ctx* ctx, const SweepShape& sh, int nbb, int 
 #undef BTE_STAGED_FM
         return;
     }
-    bte::SweepPlan spl = sp;
+    bte::SweepPlan spl{ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_dg.as<double>(), ctx->p_vo.as<double>(),
+                       ctx->p_nb.as<int>(), ctx->p_fc.as<double>(), ctx->p_lvl.as<int>(), ctx->p_lvl_off.as<int>(),
+                       ctx->n, ctx->F, ctx->n2};
     if (sh.split) {  // the same kernel over the levels split into slices of cap positions
         const StageList* sl = ctx->stage_lists.find(sh.cap)->second.get();
         spl.lvl = sl->stages.as<int>();
@@ -1838,6 +2067,45 @@ static void launch_sweep(const bte_ctx* ctx, const SweepShape& sh, int nbb, int 
     else if (fm == 3) BTE_SWEEP_FM(3);
     else BTE_SWEEP_FM(4);
 #undef BTE_SWEEP_FM
+}
+
+// Stage bounds of the stream kernel in rows: the levels, wider ones in slices
+// of at most cap positions.
+static bte_status stream_list(bte_ctx* ctx, int cap) {
+    if (ctx->stream_lists.count(cap)) return BTE_OK;
+    std::vector<int> stages, off(ctx->n_dir + 1, 0);
+    stages.reserve(ctx->plan_lrow.size());
+    for (int d = 0; d < ctx->n_dir; ++d) {
+        off[d] = (int)stages.size();
+        const int l1 = ctx->plan_lvl_off[d + 1] - 1;
+        for (int l = ctx->plan_lvl_off[d]; l < l1; ++l)
+            for (int r = ctx->plan_lrow[l]; r < ctx->plan_lrow[l + 1]; r += cap / 32) stages.push_back(r);
+        stages.push_back(ctx->plan_lrow[l1]);
+    }
+    off[ctx->n_dir] = (int)stages.size();
+    auto sl = std::make_unique<StageList>();
+    BTE_CUDA(upload(sl->stages, stages, ctx->stream));
+    BTE_CUDA(upload(sl->off, off, ctx->stream));
+    BTE_CUDA(cudaStreamSynchronize(ctx->stream));  // the host arrays go out of scope
+    ctx->stream_lists.emplace(cap, std::move(sl));
+    return BTE_OK;
+}
+
+// What a launch of shape sh reads: its plan, stage lists and records.
+static bte_status prepare_shape(bte_ctx* ctx, const SweepShape& sh) {
+    if (sh.stream) {
+        bte_status s = stream_plan(ctx);
+        if (s == BTE_OK) s = stream_list(ctx, sh.cap);
+        return s == BTE_OK ? stream_records(ctx, sh) : s;
+    }
+    bte_status s = level_plan(ctx);
+    if (s != BTE_OK) return s;
+    if (sh.kind() != 0) {
+        const StageList* sl = nullptr;
+        s = stage_list(ctx, sh.cap, &sl);
+        if (s != BTE_OK) return s;
+    }
+    return sh.staged ? staged_records(ctx) : BTE_OK;
 }
 
 // Solve all systems of one batch by upwind sweeps (exact in one sweep when no
@@ -1862,10 +2130,7 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
                        src, ctx->d_bcell.as<int>(), ctx->nbcell, ctx->d_kb.as<double>(), ctx->p_binvd.as<double>(),
                        nbb, b0, ctx->d_bsum.as<double>()));
     }
-    const bte::SweepSrc ssrc{ctx->d_ebar.as<double>(), ctx->d_bsum.as<double>(), ctx->e_prev, ctx->nbcell};
-    bte::SweepPlan sp{ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_dg.as<double>(), ctx->p_vo.as<double>(), ctx->p_nb.as<int>(),
-                      ctx->p_fc.as<double>(), ctx->p_lvl.as<int>(), ctx->p_lvl_off.as<int>(), ctx->n, ctx->F,
-                      ctx->n2};
+    const bte::SweepSrc ssrc{ctx->d_T.as<double>(), ctx->T_ref, ctx->d_bsum.as<double>(), ctx->e_prev, ctx->nbcell};
     // launch-shape autotuning on the first sweep of this plan (each candidate
     // computes the same x from the same inputs); the choice is kept per
     // process for the same device and plan shape, so a new context on the
@@ -1875,6 +2140,14 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
     const int only_shape = sweep_shape_restriction();
     const SweepTuneKey tkey{ctx->device, ctx->n, ctx->F, ctx->n_dir, nbb, ctx->plan_levels, only_margin, only_kernel,
                             only_shape};
+    // the stream kernel, unless the environment asks for another one or this
+    // plan does not suit it
+    if (!ctx->sweep_tuned && only_margin < 0 && only_shape < 0 && (only_kernel < 0 || only_kernel == 3)) {
+        bool found = false;
+        bte_status s2 = stream_choose(ctx, nbb, &found);
+        if (s2 != BTE_OK) return s2;
+        ctx->sweep_tuned = found;
+    }
     if (!ctx->sweep_tuned) {
         std::lock_guard<std::mutex> lock(g_sweep_tune_mutex);
         auto hit = g_sweep_tune.find(tkey);
@@ -1895,13 +2168,12 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
         BTE_CUDA(cudaEventCreate(&e1));
         float best = 1e30f;
         for (size_t k = 0; k < cand.size(); ++k) {
-            if (cand[k].staged || cand[k].split) {
-                const StageList* sl = nullptr;
-                bte_status s2 = stage_list(ctx, cand[k].cap, &sl);
+            {
+                bte_status s2 = prepare_shape(ctx, cand[k]);
                 if (s2 != BTE_OK) return s2;
             }
             BTE_CUDA(cudaEventRecord(e0, st));
-            launch_sweep<false>(ctx, cand[k], nbb, b0, st, sp, ssrc, 1, nullptr);
+            launch_sweep<false>(ctx, cand[k], nbb, b0, st, ssrc, 1, nullptr);
             BTE_LAUNCHED();
             BTE_CUDA(cudaEventRecord(e1, st));
             BTE_CUDA(cudaEventSynchronize(e1));
@@ -1918,7 +2190,7 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
         // margin only when that saves 3 % of the sweeps and reduction, so a
         // near tie (2D meshes) does not flip between runs.
         bool fuse = false;
-        if (ctx->plan_lagged_dirs == 0 && !ctx->sweep_shape.staged) {  // (the staged kernel leaves it to k_reduce)
+        if (ctx->plan_lagged_dirs == 0 && !ctx->sweep_shape.staged && !ctx->sweep_shape.stream) {  // (the staged kernel leaves it to k_reduce)
             if (only_margin >= 0) fuse = only_margin == 1;
             else {
                 auto time_best = [&](auto&& launch) -> float {
@@ -1936,9 +2208,9 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
                 };
                 const SweepShape sh = ctx->sweep_shape;
                 const int NB = ctx->n_band, nred = (int)(ctx->Np / bte::THREADS);
-                const float sf = time_best([&] { launch_sweep<false>(ctx, sh, nbb, b0, st, sp, ssrc, 1, nullptr); });
+                const float sf = time_best([&] { launch_sweep<false>(ctx, sh, nbb, b0, st, ssrc, 1, nullptr); });
                 const float sm = time_best(
-                    [&] { launch_sweep<true>(ctx, sh, nbb, b0, st, sp, ssrc, 1, ctx->d_spart.as<double>()); });
+                    [&] { launch_sweep<true>(ctx, sh, nbb, b0, st, ssrc, 1, ctx->d_spart.as<double>()); });
                 auto reduce = [&](bool with_margin) {
                     if (with_margin)
                         bte::k_reduce<true><<<dim3(nred, NB), bte::THREADS, 0, st>>>(
@@ -1964,12 +2236,11 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
         g_sweep_tune[tkey] = ctx->sweep_shape;
     }
     const SweepShape shape = ctx->sweep_shape;
-    if (shape.staged || shape.split) {  // a shape from the per-process cache: this plan's stage list may not exist yet
-        const StageList* sl = nullptr;
-        bte_status s2 = stage_list(ctx, shape.cap, &sl);
+    {  // (what this plan needs for a shape from the per-process cache may not exist yet)
+        bte_status s2 = prepare_shape(ctx, shape);
         if (s2 != BTE_OK) return s2;
     }
-    ctx->sweep_margin = shape.margin && !shape.staged && ctx->plan_lagged_dirs == 0;
+    ctx->sweep_margin = shape.margin && !shape.staged && !shape.stream && ctx->plan_lagged_dirs == 0;
     // algorithmic HBM bytes of a sweep per system and cell: V Omega / D and
     // k / D read, x written (and, with the fused margin, the previous iterate
     // read), plus the level-ordered geometry per direction; ebar and the
@@ -1980,10 +2251,10 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
     for (;;) {
         if (margin) {
             BTE_LAUNCH(KK_SWEEP, -1, sweep_bytes, 0,
-                       launch_sweep<true>(ctx, shape, nbb, b0, st, sp, ssrc, 1, ctx->d_spart.as<double>()));
+                       launch_sweep<true>(ctx, shape, nbb, b0, st, ssrc, 1, ctx->d_spart.as<double>()));
         } else {
             BTE_LAUNCH(KK_SWEEP, -1, sweep_bytes, 0,
-                       launch_sweep<false>(ctx, shape, nbb, b0, st, sp, ssrc, sweeps == 0, nullptr));
+                       launch_sweep<false>(ctx, shape, nbb, b0, st, ssrc, sweeps == 0, nullptr));
         }
         ++sweeps;
         if (ctx->plan_lagged_dirs == 0) break;
@@ -1991,7 +2262,7 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
         BTE_CUDA(ctx->p_bad.alloc(sizeof(int)));
         BTE_CUDA(cudaMemsetAsync(ctx->p_bad.p, 0, sizeof(int), st));
         BTE_LAUNCH(KK_SWEEP_RES, -1, S * N * 2 * w + geo, 0,
-                   bte::k_sweep_residual<<<grid, bte::THREADS, 0, st>>>(op, src, ctx->p_cell.as<int>(),
+                   bte::k_sweep_residual<<<grid, bte::THREADS, 0, st>>>(op, src, ctx->lo_perm.as<int>(),
                                                                         ctx->p_part.as<double>(), ctx->nchunk, ctx->n));
         bte::k_sweep_check<<<(S + 127) / 128, 128, 0, st>>>(ctx->p_part.as<double>(), S, ctx->nchunk, o.inner_tol,
                                                              ctx->p_bad.as<int>());
@@ -2192,12 +2463,12 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
     ctx->e_prev = ctx->d_e1.as<double>();
     BTE_CUDA(cudaMemsetAsync(ctx->e_curr, 0, sizeof(double) * NB * ND * Np, st));
     BTE_CUDA(cudaMemsetAsync(ctx->d_ebar.p, 0, sizeof(double) * NB * Np, st));  // cell_band_density = 0 (:92)
-    if (dsa_on) {
+    if (dsa_on || o.form == BTE_FORM_SWEEP) {
         // the source of the first outer iteration is ebar = 0, i.e. T = T_ref
         bte::dsa::k_fill<<<(unsigned)((Np + 255) / 256), 256, 0, st>>>(ctx->d_T.as<double>(), ctx->T_ref, (int)Np);
         BTE_LAUNCHED();
         // (the low-order work memory exists once its set-up is joined)
-        if (!dsa_pending) BTE_CUDA(cudaMemsetAsync(ctx->cg_stat.p, 0, sizeof(int) * 4, st));
+        if (dsa_on && !dsa_pending) BTE_CUDA(cudaMemsetAsync(ctx->cg_stat.p, 0, sizeof(int) * 4, st));
     }
     ctx->margins.clear();
     double Lr_sum = 0;
@@ -2658,7 +2929,7 @@ bte_status bte_get_level_order(bte_ctx* ctx, int d, int* perm, int* lvl, int cap
     if (!ctx->plan_ready) return fail(ctx, BTE_ERR_STATE, "bte_get_level_order: no sweep plan (solve in the sweep form first)");
     if (d < 0 || d >= ctx->n_dir) return fail(ctx, BTE_ERR_INVALID_ARGUMENT, "bte_get_level_order: direction out of range");
     BTE_CUDA(cudaSetDevice(ctx->device));
-    BTE_CUDA(cudaMemcpy(perm, ctx->p_cell.as<int>() + (size_t)d * ctx->n, sizeof(int) * ctx->n,
+    BTE_CUDA(cudaMemcpy(perm, ctx->lo_perm.as<int>() + (size_t)d * ctx->n, sizeof(int) * ctx->n,
                         cudaMemcpyDeviceToHost));
     const int l0 = ctx->plan_lvl_off[d], l1 = ctx->plan_lvl_off[d + 1];
     for (int k = 0; k < l1 - l0 && k < cap_lvl; ++k) lvl[k] = ctx->plan_lvl[l0 + k];
