@@ -3272,10 +3272,9 @@ namespace {
 
 // Device buffers of one MLP computation on M rows (batch).
 struct MlpWork {
-    DevBuf x, y, t, dy, act, dh, p1, p2, p3, part, params, wpack, wi, grad, m, v, idx, xall, yall;
-    int M = 0, nslices = 0;
+    DevBuf x, y, t, dy, act, dh, wpart, cpart, part, params, wpack, wi, grad, m, v, idx, xall, yall;
+    int M = 0;
 };
-constexpr int kRowsPerSlice = 256;
 
 #define MLP_CUDA(call)                                                                          \
     do {                                                                                        \
@@ -3290,16 +3289,15 @@ bte_status mlp_alloc(MlpWork& w, int M) {
     using bf = __nv_bfloat16;
     namespace ml = bte::mlp;
     w.M = M;
-    w.nslices = (M + kRowsPerSlice - 1) / kRowsPerSlice;
+    const int ns = (M + ml::SLICE - 1) / ml::SLICE, nc = (M + ml::CSLICE - 1) / ml::CSLICE;
     MLP_CUDA(w.x.alloc(sizeof(bf) * (size_t)M * ml::IN_PAD));
     MLP_CUDA(w.y.alloc(sizeof(float) * M));
     MLP_CUDA(w.t.alloc(sizeof(float) * M));
     MLP_CUDA(w.dy.alloc(sizeof(float) * M));
     MLP_CUDA(w.act.alloc(sizeof(bf) * 3 * (size_t)M * ml::H));
     MLP_CUDA(w.dh.alloc(sizeof(bf) * 3 * (size_t)M * ml::H));
-    MLP_CUDA(w.p1.alloc(sizeof(float) * (size_t)w.nslices * ml::IN_PAD * ml::H));
-    MLP_CUDA(w.p2.alloc(sizeof(float) * (size_t)w.nslices * ml::H * ml::H));
-    MLP_CUDA(w.p3.alloc(sizeof(float) * (size_t)w.nslices * ml::H * ml::H));
+    MLP_CUDA(w.wpart.alloc(sizeof(float) * (size_t)ns * ml::WPART));
+    MLP_CUDA(w.cpart.alloc(sizeof(double) * (size_t)nc * ml::CPART));
     MLP_CUDA(w.part.alloc(sizeof(double) * 256));
     MLP_CUDA(w.params.alloc(sizeof(float) * ml::NPARAM));
     MLP_CUDA(w.wpack.alloc(sizeof(bf) * ml::PK_N));
@@ -3308,6 +3306,7 @@ bte_status mlp_alloc(MlpWork& w, int M) {
     MLP_CUDA(cudaFuncSetAttribute(ml::k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ml::FWD_SMEM));
     MLP_CUDA(cudaFuncSetAttribute(ml::k_backward_data, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ml::BWD_SMEM));
+    MLP_CUDA(cudaFuncSetAttribute(ml::k_grad_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ml::GRAD_SMEM));
     return BTE_OK;
 }
 
@@ -3316,8 +3315,8 @@ int mlp_blocks(int M) { return std::max(1, std::min(1024, (M + 63) / 64)); }
 // Pack the FP32 parameters in w.params into the kernels' BF16 layouts.
 bte_status mlp_pack(MlpWork& w, cudaStream_t st) {
     namespace ml = bte::mlp;
-    ml::k_pack<<<(ml::H * ml::H + 255) / 256, 256, 0, st>>>(w.params.as<float>(), w.wpack.as<__nv_bfloat16>());
-    ml::k_pack_in_major<<<(ml::H * ml::H + 255) / 256, 256, 0, st>>>(w.params.as<float>(), w.wi.as<__nv_bfloat16>());
+    ml::k_pack<<<(ml::H * ml::H + 255) / 256, 256, 0, st>>>(w.params.as<float>(), w.wpack.as<__nv_bfloat16>(),
+                                                           w.wi.as<__nv_bfloat16>());
     MLP_CUDA(cudaGetLastError());
     return BTE_OK;
 }
@@ -3332,18 +3331,12 @@ bte_status mlp_loss_grad(MlpWork& w, int M, cudaStream_t st, double* loss) {
     ml::k_loss<<<lb, 256, 0, st>>>(w.y.as<float>(), w.t.as<float>(), M, w.dy.as<float>(), w.part.as<double>());
     ml::k_backward_data<<<mlp_blocks(M), 128, ml::BWD_SMEM, st>>>(w.dy.as<float>(), M, w.act.as<bf>(),
                                                                  w.wi.as<bf>(), w.params.as<float>(), w.dh.as<bf>());
-    const int ns = (M + kRowsPerSlice - 1) / kRowsPerSlice;
-    ml::k_weight_grad<ml::IN_PAD><<<ns, 256, 0, st>>>(w.x.as<bf>(), ml::IN_PAD, w.dh.as<bf>(), M, kRowsPerSlice,
-                                                       w.p1.as<float>());
-    ml::k_weight_grad<ml::H><<<ns, 256, 0, st>>>(w.act.as<bf>(), ml::H, w.dh.as<bf>() + (size_t)M * ml::H, M,
-                                                 kRowsPerSlice, w.p2.as<float>());
-    ml::k_weight_grad<ml::H><<<ns, 256, 0, st>>>(w.act.as<bf>() + (size_t)M * ml::H, ml::H,
-                                                 w.dh.as<bf>() + (size_t)2 * M * ml::H, M, kRowsPerSlice,
-                                                 w.p3.as<float>());
-    ml::k_grad_assemble<<<(ml::NPARAM + 255) / 256, 256, 0, st>>>(w.p1.as<float>(), w.p2.as<float>(),
-                                                                   w.p3.as<float>(), ns, w.act.as<bf>(),
-                                                                   w.dh.as<bf>(), w.dy.as<float>(), M,
-                                                                   w.grad.as<float>());
+    const int ns = (M + ml::SLICE - 1) / ml::SLICE, nc = (M + ml::CSLICE - 1) / ml::CSLICE;
+    ml::k_grad_parts<<<ml::WBLOCKS * ns + 4 * nc, 256, ml::GRAD_SMEM, st>>>(
+        w.x.as<bf>(), w.act.as<bf>(), w.dh.as<bf>(), w.dy.as<float>(), M, ns, w.wpart.as<float>(),
+        w.cpart.as<double>());
+    ml::k_grad_assemble<<<ml::ASM_BLOCKS, 256, 0, st>>>(w.wpart.as<float>(), w.cpart.as<double>(), ns, nc,
+                                                       w.grad.as<float>());
     MLP_CUDA(cudaGetLastError());
     if (loss) {
         std::vector<double> part(lb);
@@ -3391,7 +3384,7 @@ bte_status bte_set_mlp(bte_ctx* ctx, const float* params) {
     BTE_CUDA(ctx->d_wpack.alloc(sizeof(__nv_bfloat16) * ml::PK_N));
     BTE_CUDA(cudaMemcpyAsync(ctx->d_params.p, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, ctx->stream));
     ml::k_pack<<<(ml::H * ml::H + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_params.as<float>(),
-                                                                     ctx->d_wpack.as<__nv_bfloat16>());
+                                                                     ctx->d_wpack.as<__nv_bfloat16>(), nullptr);
     BTE_LAUNCHED();
     BTE_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->has_mlp = true;

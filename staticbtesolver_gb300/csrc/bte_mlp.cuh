@@ -45,8 +45,9 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// FP32 master parameters -> BF16 out-major weights.
-__global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* __restrict__ w) {
+// FP32 master parameters -> BF16 out-major weights w and, unless null, the
+// [in][out] copies of W2 and W3 that k_backward_data reads, wi[2][128][128].
+__global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wi) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < H * IN_PAD) {  // w1t[o][k]
         const int o = i / IN_PAD, k = i % IN_PAD;
@@ -56,6 +57,10 @@ __global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* __restrict__ 
         const int o = i / H, k = i % H;
         w[PK_W2 + i] = __float2bfloat16(p[OFF_W2 + k * H + o]);
         w[PK_W3 + i] = __float2bfloat16(p[OFF_W3 + k * H + o]);
+        if (wi) {
+            wi[i] = __float2bfloat16(p[OFF_W2 + i]);
+            wi[H * H + i] = __float2bfloat16(p[OFF_W3 + i]);
+        }
     }
     if (i < 8 * H) {
         const int o = i / H, k = i % H;
@@ -63,16 +68,30 @@ __global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* __restrict__ 
     }
 }
 
-// Shared-memory image of the packed weights and the biases.
+// Shared-memory image of the packed weights and the biases.  Rows are 16 bytes
+// longer than they are full, so that the eight rows of an 8 x 8 fragment lie in
+// different banks (rows of 256 bytes: all in one, eight turns for each load).
+// With that, 16-byte copies and ldmatrix the forward pass of 4,096 rows takes
+// 10 us (before: 30), the backward one 12 (45).
+constexpr int LD1 = IN_PAD + 8, LD = H + 8;
 struct Smem {
-    __nv_bfloat16 w[PK_N];
+    __nv_bfloat16 w1[H * LD1], w2[H * LD], w3[H * LD], w4[8 * LD];
     float b[3 * H + 1];
 };
 
+// rows of `vec` 16-byte words -> shared memory rows of ld elements
+__device__ __forceinline__ void load_rows(__nv_bfloat16* dst, int ld, const __nv_bfloat16* __restrict__ src, int rows,
+                                          int vec) {
+    const uint4* g = reinterpret_cast<const uint4*>(src);
+    for (int i = threadIdx.x; i < rows * vec; i += blockDim.x)
+        *reinterpret_cast<uint4*>(dst + (size_t)(i / vec) * ld + 8 * (i % vec)) = g[i];
+}
+
 __device__ __forceinline__ void load_smem(Smem& s, const __nv_bfloat16* __restrict__ w, const float* __restrict__ p) {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(w);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(s.w);
-    for (int i = threadIdx.x; i < PK_N / 2; i += blockDim.x) dst[i] = src[i];
+    load_rows(s.w1, LD1, w + PK_W1, H, IN_PAD / 8);
+    load_rows(s.w2, LD, w + PK_W2, H, H / 8);
+    load_rows(s.w3, LD, w + PK_W3, H, H / 8);
+    load_rows(s.w4, LD, w + PK_W4, 8, H / 8);
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         s.b[i] = p[OFF_B1 + i];
         s.b[H + i] = p[OFF_B2 + i];
@@ -82,21 +101,38 @@ __device__ __forceinline__ void load_smem(Smem& s, const __nv_bfloat16* __restri
     __syncthreads();
 }
 
-// One hidden layer for this warp's 16 rows: acc = A(16 x K) * W^T, K = 16*kt.
-// wt is [128][ldk] out-major; a[kk] are the A fragments of k-tile kk.
-template <int KT>
-__device__ __forceinline__ void layer(float (&acc)[16][4], const uint32_t (&a)[KT][4], const __nv_bfloat16* wt, int ldk,
-                                      int g, int t) {
+// Four 8 x 8 tiles of 16-bit elements; lane l gives the address of row l % 8 of
+// tile l / 8 (16-byte aligned).
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const __nv_bfloat16* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
+}
+
+// 8 output columns (rows of wt) of A(16 x 128) * W^T, added to c.
+__device__ __forceinline__ void columns8(float (&c)[4], const uint32_t (&a)[8][4], const __nv_bfloat16* wt, int lane) {
+    const __nv_bfloat16* row = wt + (size_t)(lane & 7) * LD + 8 * (lane >> 3);
+#pragma unroll
+    for (int kk = 0; kk < 8; kk += 2) {
+        uint32_t b[4];
+        ldsm4(b, row + 16 * kk);
+        mma16816(c, a[kk], b[0], b[1]);
+        mma16816(c, a[kk + 1], b[2], b[3]);
+    }
+}
+
+// One hidden layer for this warp's 16 rows: acc = A(16 x 128) * W^T, wt out-major.
+__device__ __forceinline__ void layer(float (&acc)[16][4], const uint32_t (&a)[8][4], const __nv_bfloat16* wt,
+                                      int lane) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-        const __nv_bfloat16* row = wt + (size_t)(8 * j + g) * ldk + 2 * t;
-#pragma unroll
-        for (int kk = 0; kk < KT; ++kk) {
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(row + 16 * kk);
-            const uint32_t b1 = *reinterpret_cast<const uint32_t*>(row + 16 * kk + 8);
-            mma16816(acc[j], a[kk], b0, b1);
-        }
+        columns8(acc[j], a, wt + (size_t)8 * j * LD, lane);
     }
 }
 
@@ -160,23 +196,22 @@ __global__ void __launch_bounds__(128) k_forward(const __nv_bfloat16* __restrict
         }
         float acc[16][4];
         uint32_t h[8][4];
-        layer<1>(acc, a1, s.w + PK_W1, IN_PAD, g, t);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+            const uint32_t* b = reinterpret_cast<const uint32_t*>(s.w1 + (size_t)(8 * j + g) * LD1 + 2 * t);
+            mma16816(acc[j], a1[0], b[0], b[4]);
+        }
         relu_pack(acc, s.b, t, h);
         if (act) store_frag(h, act, r0, g, t, M);
-        layer<8>(acc, h, s.w + PK_W2, H, g, t);
+        layer(acc, h, s.w2, lane);
         relu_pack(acc, s.b + H, t, h);
         if (act) store_frag(h, act + (size_t)M * H, r0, g, t, M);
-        layer<8>(acc, h, s.w + PK_W3, H, g, t);
+        layer(acc, h, s.w3, lane);
         relu_pack(acc, s.b + 2 * H, t, h);
         if (act) store_frag(h, act + (size_t)2 * M * H, r0, g, t, M);
         float o[4] = {0, 0, 0, 0};
-        const __nv_bfloat16* row = s.w + PK_W4 + (size_t)g * H + 2 * t;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(row + 16 * kk);
-            const uint32_t b1 = *reinterpret_cast<const uint32_t*>(row + 16 * kk + 8);
-            mma16816(o, h[kk], b0, b1);
-        }
+        columns8(o, h, s.w4, lane);
         if (t == 0) {  // column 0 of the 16 x 8 output tile
             if (r0 + g < M) y[r0 + g] = o[0] + s.b[3 * H];
             if (r0 + g + 8 < M) y[r0 + g + 8] = o[2] + s.b[3 * H];
@@ -215,55 +250,51 @@ __global__ void __launch_bounds__(128) k_backward_data(const float* __restrict__
                                                        const float* __restrict__ p, __nv_bfloat16* __restrict__ dh) {
     extern __shared__ __align__(16) unsigned char smem_bwd[];  // BWD_SMEM bytes
     __nv_bfloat16* sw = reinterpret_cast<__nv_bfloat16*>(smem_bwd);
-    float* w4 = reinterpret_cast<float*>(smem_bwd + sizeof(__nv_bfloat16) * 2 * H * H);
-    {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(wi);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(sw);
-        for (int i = threadIdx.x; i < H * H; i += blockDim.x) dst[i] = src[i];
-        for (int i = threadIdx.x; i < H; i += blockDim.x) w4[i] = p[OFF_W4 + i];
-        __syncthreads();
-    }
+    float* w4 = reinterpret_cast<float*>(smem_bwd + sizeof(__nv_bfloat16) * 2 * H * LD);
+    load_rows(sw, LD, wi, 2 * H, H / 8);
+    for (int i = threadIdx.x; i < H; i += blockDim.x) w4[i] = p[OFF_W4 + i];
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int nwarps = gridDim.x * (blockDim.x >> 5);
     for (int r0 = (blockIdx.x * (blockDim.x >> 5) + warp) * 16; r0 < M; r0 += nwarps * 16) {
         const int ra = r0 + g, rb = r0 + g + 8;
         const float dya = ra < M ? dy[ra] : 0.0f, dyb = rb < M ? dy[rb] : 0.0f;
-        auto act_at = [&](int layer_i, int r, int c) -> float {
-            return r < M ? __bfloat162float(act[((size_t)layer_i * M + r) * H + c]) : 0.0f;
+        // activations of columns c, c + 1 (c even) of row r, 0 beyond the last row
+        auto act2 = [&](int layer_i, int r, int c) -> float2 {
+            const uint32_t v =
+                r < M ? *reinterpret_cast<const uint32_t*>(act + ((size_t)layer_i * M + r) * H + c) : 0u;
+            return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
         };
         // dh3 in A-fragment form directly
         uint32_t d[8][4];
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
-            const int c0 = 16 * kk + 2 * t, c1 = c0 + 8;
-            float v[8];
-            v[0] = act_at(2, ra, c0) > 0.f ? dya * w4[c0] : 0.f;
-            v[1] = act_at(2, ra, c0 + 1) > 0.f ? dya * w4[c0 + 1] : 0.f;
-            v[2] = act_at(2, rb, c0) > 0.f ? dyb * w4[c0] : 0.f;
-            v[3] = act_at(2, rb, c0 + 1) > 0.f ? dyb * w4[c0 + 1] : 0.f;
-            v[4] = act_at(2, ra, c1) > 0.f ? dya * w4[c1] : 0.f;
-            v[5] = act_at(2, ra, c1 + 1) > 0.f ? dya * w4[c1 + 1] : 0.f;
-            v[6] = act_at(2, rb, c1) > 0.f ? dyb * w4[c1] : 0.f;
-            v[7] = act_at(2, rb, c1 + 1) > 0.f ? dyb * w4[c1 + 1] : 0.f;
-            d[kk][0] = pack2(v[0], v[1]);
-            d[kk][1] = pack2(v[2], v[3]);
-            d[kk][2] = pack2(v[4], v[5]);
-            d[kk][3] = pack2(v[6], v[7]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = 16 * kk + 2 * t + 8 * (q >> 1);
+                const float2 h = act2(2, q & 1 ? rb : ra, c);
+                const float dq = q & 1 ? dyb : dya;
+                d[kk][q] = pack2(h.x > 0.f ? dq * w4[c] : 0.f, h.y > 0.f ? dq * w4[c + 1] : 0.f);
+            }
         }
         store_frag(d, dh + (size_t)2 * M * H, r0, g, t, M);
         // dh2 = dh3 W3^T, then dh1 = dh2 W2^T; masks from h2, h1
         for (int li = 1; li >= 0; --li) {
-            float acc[16][4];
-            layer<8>(acc, d, sw + (size_t)li * H * H, H, g, t);  // B[k=out][n=in] = W[in][out]: rows of wi are "in"
+            uint64_t off = 0;  // bit 4 j + i: acc[j][i] belongs to an inactive unit
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                const int c = 8 * j + 2 * t;
-                if (act_at(li, ra, c) <= 0.f) acc[j][0] = 0.f;
-                if (act_at(li, ra, c + 1) <= 0.f) acc[j][1] = 0.f;
-                if (act_at(li, rb, c) <= 0.f) acc[j][2] = 0.f;
-                if (act_at(li, rb, c + 1) <= 0.f) acc[j][3] = 0.f;
+                const float2 ha = act2(li, ra, 8 * j + 2 * t), hb = act2(li, rb, 8 * j + 2 * t);
+                off |= (uint64_t)((ha.x <= 0.f) | (ha.y <= 0.f) << 1 | (hb.x <= 0.f) << 2 | (hb.y <= 0.f) << 3)
+                       << (4 * j);
             }
+            float acc[16][4];
+            layer(acc, d, sw + (size_t)li * H * LD, lane);  // B[k=out][n=in] = W[in][out]: rows of wi are "in"
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (off >> (4 * j + i) & 1) acc[j][i] = 0.f;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 d[kk][0] = pack2(acc[2 * kk][0], acc[2 * kk][1]);
@@ -277,117 +308,168 @@ __global__ void __launch_bounds__(128) k_backward_data(const float* __restrict__
 }
 
 constexpr size_t FWD_SMEM = sizeof(Smem);
-constexpr size_t BWD_SMEM = sizeof(__nv_bfloat16) * 2 * H * H + sizeof(float) * H;
+constexpr size_t BWD_SMEM = sizeof(__nv_bfloat16) * 2 * H * LD + sizeof(float) * H;
 
-// FP32 master weights -> BF16 [in][out] copies of W2 and W3 for k_backward_data.
-__global__ void k_pack_in_major(const float* __restrict__ p, __nv_bfloat16* __restrict__ wi) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= H * H) return;
-    wi[i] = __float2bfloat16(p[OFF_W2 + i]);
-    wi[H * H + i] = __float2bfloat16(p[OFF_W3 + i]);
+// Sums over the rows of the batch, in slices, for k_grad_assemble:
+//   wpart[slice][W1 16 x 128 | W2 128 x 128 | W3 128 x 128], in-major,
+//       = sum over the slice's SLICE rows of a[r][in] d[r][out] (FP32, tensor cores);
+//   cpart[column slice][dh1 | dh2 | dh3 | h3 dy | dy], 4 x 128 + 1 values,
+//       = sums over its CSLICE rows (FP64).
+//
+// All of it in one launch: per slice of rows one block for W1 and four for each
+// of W2 and W3 (a 64 x 64 quadrant), per column slice one for each of the four
+// column sums.  The column sums are what bounds it: every value takes an FP64
+// conversion and addition, 19 cycles of an SM's pipe per warp, so they have
+// short slices and blocks of their own that fill the chip.  One thread per bias
+// going through all rows, as they were before, took 880 us for 4,096 rows, and
+// the three weight gradients 114; now 24 us together, and 5 for the assembly.
+// The rows of a tile come by cp.async in four groups of 64, and its fragments
+// by ldmatrix with transposition, both operands being row-major in the batch.
+constexpr int SLICE = 256, CSLICE = 64;
+constexpr int WPART = IN_PAD * H + 2 * H * H, CPART = 4 * H + 1;
+constexpr int WBLOCKS = 9;               // blocks per slice
+constexpr int QLD = 64 + 8;              // row of a quadrant's operand tile
+constexpr size_t GRAD_SMEM = sizeof(__nv_bfloat16) * SLICE * (LD1 + LD);  // W1's; a quadrant needs 2 QLD a row
+static_assert(2 * QLD <= LD1 + LD, "operand tiles of a quadrant fit");
+
+__device__ __forceinline__ void cp16(__nv_bfloat16* dst, const __nv_bfloat16* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(valid ? 16 : 0));
 }
 
-// Weight gradients for one layer over a slice of rows:
-//   part[slice][in][out] = sum_{rows of slice} a[r][in] * d[r][out]
-// a: [M][lda] bf16 (lda = 16 for the input layer, 128 otherwise), d: [M][128]
-// bf16.  Block = 8 warps; warp w owns in-rows 16*(w % (KIN/16)) .. and out
-// columns 64*(w / (KIN/16)) ...  The transposed A operand is staged through
-// shared memory.  Rows are taken in slices of 64.
-template <int KIN>
-__global__ void __launch_bounds__(256) k_weight_grad(const __nv_bfloat16* __restrict__ a, int lda,
-                                                     const __nv_bfloat16* __restrict__ d, int M, int rows_per_slice,
-                                                     float* __restrict__ part) {
-    __shared__ __align__(16) __nv_bfloat16 sa[64][KIN + 8];
-    __shared__ __align__(16) __nv_bfloat16 sd[64][H + 8];
+// out[in][out] of a tile: KIN in-columns of a (row length lda) and NOUT
+// out-columns of d, rows r0 .. r1 - 1 (at most SLICE); warp w of 8 has in-columns
+// 16 (w % (KIN / 16)) and an equal share of the out-columns.
+template <int KIN, int NOUT, int SA, int SD>
+__device__ __forceinline__ void weight_tile(const __nv_bfloat16* __restrict__ a, int lda,
+                                            const __nv_bfloat16* __restrict__ d, int r0, int r1, float* out,
+                                            __nv_bfloat16* sa) {
+    __nv_bfloat16* sd = sa + SLICE * SA;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    constexpr int MT = KIN / 16;          // 16-row tiles of "in"
-    constexpr int NW_OUT = 8 / MT;        // warps sharing one in-tile
-    const int mt = warp % MT;
-    constexpr int n_span = H / NW_OUT;    // out columns per warp
-    const int n0 = (warp / MT) * n_span;
-    float acc[16][4];
+    constexpr int MT = KIN / 16, SPAN = NOUT / (8 / MT);
+    const int m0 = 16 * (warp % MT), n0 = SPAN * (warp / MT);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    const int r_begin = blockIdx.x * rows_per_slice;
-    const int r_end = min(M, r_begin + rows_per_slice);
-    for (int rb = r_begin; rb < r_end; rb += 64) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < 64 * KIN; i += blockDim.x) {
-            const int r = i / KIN, c = i % KIN;
-            sa[r][c] = (rb + r < r_end) ? a[(size_t)(rb + r) * lda + c] : __float2bfloat16(0.f);
+    for (int q = 0; q < 4; ++q) {
+        for (int i = threadIdx.x; i < 64 * (KIN + NOUT) / 8; i += 256) {
+            const int r = 64 * q + i / ((KIN + NOUT) / 8), c = i % ((KIN + NOUT) / 8) * 8;
+            const bool in = r0 + r < r1;
+            const size_t row = in ? r0 + r : r0;  // (rows beyond the end read as zero)
+            if (c < KIN) cp16(sa + r * SA + c, a + row * lda + c, in);
+            else cp16(sd + r * SD + c - KIN, d + row * H + c - KIN, in);
         }
-        for (int i = threadIdx.x; i < 64 * H; i += blockDim.x) {
-            const int r = i / H, c = i % H;
-            sd[r][c] = (rb + r < r_end) ? d[(size_t)(rb + r) * H + c] : __float2bfloat16(0.f);
-        }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;\n");
+    }
+    float acc[SPAN / 8][4];
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {  // 16 rows per k-step
-            const int k0 = 16 * ks;
+    for (int j = 0; j < SPAN / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    const __nv_bfloat16* pa = sa + ((lane & 7) + 8 * (lane >> 4)) * SA + m0 + 8 * (lane >> 3 & 1);
+    const __nv_bfloat16* pd = sd + ((lane & 7) + 8 * (lane >> 3 & 1)) * SD + n0 + 8 * (lane >> 4);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q == 0) asm volatile("cp.async.wait_group 3;\n");
+        if (q == 1) asm volatile("cp.async.wait_group 2;\n");
+        if (q == 2) asm volatile("cp.async.wait_group 1;\n");
+        if (q == 3) asm volatile("cp.async.wait_group 0;\n");
+        __syncthreads();
+        if (r0 + 64 * q >= r1) continue;
+#pragma unroll
+        for (int k0 = 64 * q; k0 < 64 * q + 64; k0 += 16) {
             uint32_t af[4];
-            const int m = 16 * mt + g;
-            af[0] = pack2(sa[k0 + 2 * t][m], sa[k0 + 2 * t + 1][m]);
-            af[1] = pack2(sa[k0 + 2 * t][m + 8], sa[k0 + 2 * t + 1][m + 8]);
-            af[2] = pack2(sa[k0 + 2 * t + 8][m], sa[k0 + 2 * t + 9][m]);
-            af[3] = pack2(sa[k0 + 2 * t + 8][m + 8], sa[k0 + 2 * t + 9][m + 8]);
+            ldsm4_t(af, pa + k0 * SA);
 #pragma unroll
-            for (int j = 0; j < n_span / 8; ++j) {
-                const int n = n0 + 8 * j + g;
-                const uint32_t b0 = pack2(sd[k0 + 2 * t][n], sd[k0 + 2 * t + 1][n]);
-                const uint32_t b1 = pack2(sd[k0 + 2 * t + 8][n], sd[k0 + 2 * t + 9][n]);
-                mma16816(acc[j], af, b0, b1);
+            for (int j = 0; j < SPAN / 8; j += 2) {
+                uint32_t b[4];
+                ldsm4_t(b, pd + k0 * SD + 8 * j);
+                mma16816(acc[j], af, b[0], b[1]);
+                mma16816(acc[j + 1], af, b[2], b[3]);
             }
         }
     }
-    float* out = part + (size_t)blockIdx.x * KIN * H;
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int j = 0; j < n_span / 8; ++j) {
-        const int c = n0 + 8 * j + 2 * t;
-        const int r = 16 * mt + g;
-        out[(size_t)r * H + c] = acc[j][0];
-        out[(size_t)r * H + c + 1] = acc[j][1];
-        out[(size_t)(r + 8) * H + c] = acc[j][2];
-        out[(size_t)(r + 8) * H + c + 1] = acc[j][3];
+    for (int j = 0; j < SPAN / 8; ++j) {
+        float* o = out + (size_t)(m0 + g) * H + n0 + 8 * j + 2 * t;
+        *reinterpret_cast<float2*>(o) = make_float2(acc[j][0], acc[j][1]);
+        *reinterpret_cast<float2*>(o + 8 * H) = make_float2(acc[j][2], acc[j][3]);
     }
 }
 
-// Gradient assembly into the flat FP32 layout:
-//   weights: sum over slices of part (fixed order); W4[k] = sum_r h3[r][k] dy[r];
-//   biases: b_l[o] = sum_r dh_l[r][o]; b4 = sum_r dy[r].
-// One thread per parameter.
-__global__ void k_grad_assemble(const float* __restrict__ p1, const float* __restrict__ p2,
-                                const float* __restrict__ p3, int nslices, const __nv_bfloat16* __restrict__ act,
-                                const __nv_bfloat16* __restrict__ dh, const float* __restrict__ dy, int M,
-                                float* __restrict__ grad) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
-    double s = 0.0;
-    if (i < OFF_B1) {  // W1[k][o], part1 is [slice][16][128]
-        const int k = i / H, o = i % H;
-        for (int q = 0; q < nslices; ++q) s += p1[((size_t)q * IN_PAD + k) * H + o];
-    } else if (i < OFF_W2) {
-        const int o = i - OFF_B1;
-        for (int r = 0; r < M; ++r) s += __bfloat162float(dh[(size_t)r * H + o]);
-    } else if (i < OFF_B2) {
-        const int k = (i - OFF_W2) / H, o = (i - OFF_W2) % H;
-        for (int q = 0; q < nslices; ++q) s += p2[((size_t)q * H + k) * H + o];
-    } else if (i < OFF_W3) {
-        const int o = i - OFF_B2;
-        for (int r = 0; r < M; ++r) s += __bfloat162float(dh[((size_t)M + r) * H + o]);
-    } else if (i < OFF_B3) {
-        const int k = (i - OFF_W3) / H, o = (i - OFF_W3) % H;
-        for (int q = 0; q < nslices; ++q) s += p3[((size_t)q * H + k) * H + o];
-    } else if (i < OFF_W4) {
-        const int o = i - OFF_B3;
-        for (int r = 0; r < M; ++r) s += __bfloat162float(dh[((size_t)2 * M + r) * H + o]);
-    } else if (i < OFF_B4) {
-        const int k = i - OFF_W4;
-        for (int r = 0; r < M; ++r) s += (double)__bfloat162float(act[((size_t)2 * M + r) * H + k]) * dy[r];
-    } else {
-        for (int r = 0; r < M; ++r) s += dy[r];
+__global__ void __launch_bounds__(256) k_grad_parts(const __nv_bfloat16* __restrict__ x,
+                                                    const __nv_bfloat16* __restrict__ act,
+                                                    const __nv_bfloat16* __restrict__ dh,
+                                                    const float* __restrict__ dy, int M, int ns,
+                                                    float* __restrict__ wpart, double* __restrict__ cpart) {
+    extern __shared__ __align__(16) unsigned char smem_grad[];  // GRAD_SMEM bytes
+    const size_t L = (size_t)M * H;
+    if ((int)blockIdx.x < WBLOCKS * ns) {
+        __nv_bfloat16* sm = reinterpret_cast<__nv_bfloat16*>(smem_grad);
+        const int s = blockIdx.x / WBLOCKS, job = blockIdx.x % WBLOCKS;
+        const int r0 = s * SLICE, r1 = min(M, r0 + SLICE);
+        float* out = wpart + (size_t)s * WPART;
+        if (job == 8) {
+            weight_tile<IN_PAD, H, LD1, LD>(x, IN_PAD, dh, r0, r1, out, sm);
+        } else {
+            const int l = job >> 2, i0 = 64 * (job >> 1 & 1), o0 = 64 * (job & 1);
+            weight_tile<64, 64, QLD, QLD>(act + l * L + i0, H, dh + (l + 1) * L + o0, r0, r1,
+                                          out + IN_PAD * H + l * H * H + (size_t)i0 * H + o0, sm);
+        }
+        return;
     }
-    grad[i] = (float)s;
+    const int k = blockIdx.x - WBLOCKS * ns, s = k >> 2, q = k & 3;
+    const int r0 = s * CSLICE, r1 = min(M, r0 + CSLICE);
+    double* out = cpart + (size_t)s * CPART;
+    const __nv_bfloat16* v = (q < 3 ? dh + q * L : act + 2 * L) + 2 * (threadIdx.x & 63);
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 8
+    for (int r = r0 + (threadIdx.x >> 6); r < r1; r += 4) {
+        const uint32_t u = *reinterpret_cast<const uint32_t*>(v + (size_t)r * H);
+        const float lo = __uint_as_float(u << 16), hi = __uint_as_float(u & 0xffff0000u);
+        if (q < 3) {
+            s0 += lo;
+            s1 += hi;
+        } else {
+            const double y = dy[r];
+            s0 += (double)lo * y;
+            s1 += (double)hi * y;
+        }
+    }
+    double* red = reinterpret_cast<double*>(smem_grad);  // [4][128]
+    red[threadIdx.x * 2] = s0;
+    red[threadIdx.x * 2 + 1] = s1;
+    __syncthreads();
+    if (threadIdx.x < H)
+        out[q * H + threadIdx.x] = (red[threadIdx.x] + red[H + threadIdx.x]) + (red[2 * H + threadIdx.x] + red[3 * H + threadIdx.x]);
+    if (q == 3 && threadIdx.x >= 224) {
+        double t = 0.0;
+        for (int r = r0 + (int)threadIdx.x - 224; r < r1; r += 32) t += dy[r];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 224) out[4 * H] = t;
+    }
+}
+
+// The sums of the slices, FP64 in fixed order, into the flat FP32 gradient: one
+// thread per weight, one warp per column sum (W4, the biases).
+constexpr int ASM_WBLOCKS = (IN * H + 2 * H * H) / 256, ASM_BLOCKS = ASM_WBLOCKS + (CPART + 7) / 8;
+__global__ void __launch_bounds__(256) k_grad_assemble(const float* __restrict__ wpart,
+                                                       const double* __restrict__ cpart, int ns, int nc,
+                                                       float* __restrict__ grad) {
+    double s = 0.0;
+    if ((int)blockIdx.x < ASM_WBLOCKS) {
+        int i = blockIdx.x * 256 + threadIdx.x;
+        const int src = i < IN * H ? i : i + (IN_PAD - IN) * H;  // (W1's padding inputs are left out)
+#pragma unroll 8
+        for (int q = 0; q < ns; ++q) s += wpart[(size_t)q * WPART + src];
+        if (i >= IN * H) i += H;
+        if (i >= OFF_B2) i += H;
+        grad[i] = (float)s;
+        return;
+    }
+    const int k = (blockIdx.x - ASM_WBLOCKS) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (k >= CPART) return;
+    for (int q = lane; q < nc; q += 32) s += cpart[(size_t)q * CPART + k];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    const int at[5] = {OFF_B1, OFF_B2, OFF_B3, OFF_W4, OFF_B4};
+    if (lane == 0) grad[at[k / H] + k % H] = (float)s;
 }
 
 // Adam (Kingma & Ba) on the FP32 master parameters.
