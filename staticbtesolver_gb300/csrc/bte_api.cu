@@ -63,6 +63,28 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
+// Several device arrays in one allocation: mapping and unmapping device memory
+// costs a one-shot call more than small kernels do (the 17 arrays of a network
+// gradient of 4,096 rows: 500 us a call apart, 275 together).
+struct DevSlab {
+    DevBuf mem;
+    template <typename T>
+    void add(T*& p, size_t count) {
+        at.push_back({reinterpret_cast<void**>(&p), size});
+        size += (sizeof(T) * count + 255) / 256 * 256;
+    }
+    cudaError_t alloc() {
+        const cudaError_t e = mem.alloc(size);
+        if (e != cudaSuccess) return e;
+        for (auto& a : at) *a.first = mem.as<unsigned char>() + a.second;
+        return cudaSuccess;
+    }
+
+private:
+    std::vector<std::pair<void**, size_t>> at;
+    size_t size = 0;
+};
+
 constexpr int kGroup = 8;  // BiCGSTAB iterations launched between host checks
 
 enum KernelKind { KK_P, KK_SPMV1, KK_S, KK_SPMV2, KK_X, KK_INIT, KK_RHS, KK_REDUCE, KK_DIFFUSE, KK_HEAT, KK_SWEEP,
@@ -3270,10 +3292,17 @@ extern "C" bte_status bte_bicgstab_csr_noalloc(int n, const int* rowptr, const i
 
 namespace {
 
-// Device buffers of one MLP computation on M rows (batch).
+// Device arrays of one MLP computation on a batch of up to M rows: what the
+// forward pass takes, and (gradient) what the gradient adds to it.  Further
+// arrays of the caller's may be added to slab before alloc().
 struct MlpWork {
-    DevBuf x, y, t, dy, act, dh, wpart, cpart, part, params, wpack, wi, grad, m, v, idx, xall, yall;
-    int M = 0;
+    using bf = __nv_bfloat16;
+    DevSlab slab;
+    bf *x = nullptr, *act = nullptr, *dh = nullptr, *wpack = nullptr, *wi = nullptr;
+    float *xf = nullptr, *y = nullptr, *t = nullptr, *dy = nullptr, *wpart = nullptr, *params = nullptr, *grad = nullptr;
+    double *cpart = nullptr, *part = nullptr;
+    void arrays(size_t M, bool gradient);
+    bte_status alloc();
 };
 
 #define MLP_CUDA(call)                                                                          \
@@ -3285,24 +3314,27 @@ struct MlpWork {
         }                                                                                       \
     } while (0)
 
-bte_status mlp_alloc(MlpWork& w, int M) {
-    using bf = __nv_bfloat16;
+void MlpWork::arrays(size_t M, bool gradient) {
     namespace ml = bte::mlp;
-    w.M = M;
-    const int ns = (M + ml::SLICE - 1) / ml::SLICE, nc = (M + ml::CSLICE - 1) / ml::CSLICE;
-    MLP_CUDA(w.x.alloc(sizeof(bf) * (size_t)M * ml::IN_PAD));
-    MLP_CUDA(w.y.alloc(sizeof(float) * M));
-    MLP_CUDA(w.t.alloc(sizeof(float) * M));
-    MLP_CUDA(w.dy.alloc(sizeof(float) * M));
-    MLP_CUDA(w.act.alloc(sizeof(bf) * 3 * (size_t)M * ml::H));
-    MLP_CUDA(w.dh.alloc(sizeof(bf) * 3 * (size_t)M * ml::H));
-    MLP_CUDA(w.wpart.alloc(sizeof(float) * (size_t)ns * ml::WPART));
-    MLP_CUDA(w.cpart.alloc(sizeof(double) * (size_t)nc * ml::CPART));
-    MLP_CUDA(w.part.alloc(sizeof(double) * 256));
-    MLP_CUDA(w.params.alloc(sizeof(float) * ml::NPARAM));
-    MLP_CUDA(w.wpack.alloc(sizeof(bf) * ml::PK_N));
-    MLP_CUDA(w.wi.alloc(sizeof(bf) * 2 * ml::H * ml::H));
-    MLP_CUDA(w.grad.alloc(sizeof(float) * ml::NPARAM));
+    slab.add(x, M * ml::IN_PAD);
+    slab.add(y, M);
+    slab.add(params, ml::NPARAM);
+    slab.add(wpack, ml::PK_N);
+    if (!gradient) return;
+    slab.add(t, M);
+    slab.add(dy, M);
+    slab.add(act, 3 * M * ml::H);
+    slab.add(dh, 3 * M * ml::H);
+    slab.add(wpart, (M + ml::SLICE - 1) / ml::SLICE * ml::WPART);
+    slab.add(cpart, (M + ml::CSLICE - 1) / ml::CSLICE * ml::CPART);
+    slab.add(part, 256);
+    slab.add(wi, 2 * ml::H * ml::H);
+    slab.add(grad, ml::NPARAM);
+}
+
+bte_status MlpWork::alloc() {
+    namespace ml = bte::mlp;
+    MLP_CUDA(slab.alloc());
     MLP_CUDA(cudaFuncSetAttribute(ml::k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ml::FWD_SMEM));
     MLP_CUDA(cudaFuncSetAttribute(ml::k_backward_data, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ml::BWD_SMEM));
@@ -3315,8 +3347,7 @@ int mlp_blocks(int M) { return std::max(1, std::min(1024, (M + 63) / 64)); }
 // Pack the FP32 parameters in w.params into the kernels' BF16 layouts.
 bte_status mlp_pack(MlpWork& w, cudaStream_t st) {
     namespace ml = bte::mlp;
-    ml::k_pack<<<(ml::H * ml::H + 255) / 256, 256, 0, st>>>(w.params.as<float>(), w.wpack.as<__nv_bfloat16>(),
-                                                           w.wi.as<__nv_bfloat16>());
+    ml::k_pack<<<(ml::H * ml::H + 255) / 256, 256, 0, st>>>(w.params, w.wpack, w.wi);
     MLP_CUDA(cudaGetLastError());
     return BTE_OK;
 }
@@ -3325,22 +3356,18 @@ bte_status mlp_pack(MlpWork& w, cudaStream_t st) {
 bte_status mlp_loss_grad(MlpWork& w, int M, cudaStream_t st, double* loss) {
     namespace ml = bte::mlp;
     using bf = __nv_bfloat16;
-    ml::k_forward<<<mlp_blocks(M), 128, ml::FWD_SMEM, st>>>(w.x.as<bf>(), M, w.wpack.as<bf>(), w.params.as<float>(),
-                                                          w.y.as<float>(), w.act.as<bf>());
+    ml::k_forward<<<mlp_blocks(M), 128, ml::FWD_SMEM, st>>>(w.x, M, w.wpack, w.params, w.y, w.act);
     const int lb = std::min(256, (M + 255) / 256);
-    ml::k_loss<<<lb, 256, 0, st>>>(w.y.as<float>(), w.t.as<float>(), M, w.dy.as<float>(), w.part.as<double>());
-    ml::k_backward_data<<<mlp_blocks(M), 128, ml::BWD_SMEM, st>>>(w.dy.as<float>(), M, w.act.as<bf>(),
-                                                                 w.wi.as<bf>(), w.params.as<float>(), w.dh.as<bf>());
+    ml::k_loss<<<lb, 256, 0, st>>>(w.y, w.t, M, w.dy, w.part);
+    ml::k_backward_data<<<mlp_blocks(M), 128, ml::BWD_SMEM, st>>>(w.dy, M, w.act, w.wi, w.params, w.dh);
     const int ns = (M + ml::SLICE - 1) / ml::SLICE, nc = (M + ml::CSLICE - 1) / ml::CSLICE;
     ml::k_grad_parts<<<ml::WBLOCKS * ns + 4 * nc, 256, ml::GRAD_SMEM, st>>>(
-        w.x.as<bf>(), w.act.as<bf>(), w.dh.as<bf>(), w.dy.as<float>(), M, ns, w.wpart.as<float>(),
-        w.cpart.as<double>());
-    ml::k_grad_assemble<<<ml::ASM_BLOCKS, 256, 0, st>>>(w.wpart.as<float>(), w.cpart.as<double>(), ns, nc,
-                                                       w.grad.as<float>());
+        w.x, w.act, w.dh, w.dy, M, ns, w.wpart, w.cpart);
+    ml::k_grad_assemble<<<ml::ASM_BLOCKS, 256, 0, st>>>(w.wpart, w.cpart, ns, nc, w.grad);
     MLP_CUDA(cudaGetLastError());
     if (loss) {
         std::vector<double> part(lb);
-        MLP_CUDA(cudaMemcpyAsync(part.data(), w.part.p, sizeof(double) * lb, cudaMemcpyDeviceToHost, st));
+        MLP_CUDA(cudaMemcpyAsync(part.data(), w.part, sizeof(double) * lb, cudaMemcpyDeviceToHost, st));
         MLP_CUDA(cudaStreamSynchronize(st));
         double s = 0;
         for (double v : part) s += v;
@@ -3407,19 +3434,18 @@ bte_status bte_mlp_predict(const float* X, int M, const float* params, float* y)
     ScopedStream ss;
     MLP_CUDA(cudaStreamCreateWithFlags(&ss.s, cudaStreamNonBlocking));
     MlpWork w;
-    bte_status rc = mlp_alloc(w, M);
+    w.arrays(M, false);
+    w.slab.add(w.xf, (size_t)M * ml::IN);
+    bte_status rc = w.alloc();
     if (rc) return rc;
-    DevBuf xf;
-    MLP_CUDA(xf.alloc(sizeof(float) * (size_t)M * ml::IN));
-    MLP_CUDA(cudaMemcpyAsync(xf.p, X, sizeof(float) * (size_t)M * ml::IN, cudaMemcpyHostToDevice, ss.s));
-    MLP_CUDA(cudaMemcpyAsync(w.params.p, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, ss.s));
-    ml::k_features_bf16<<<(M * ml::IN_PAD + 255) / 256, 256, 0, ss.s>>>(xf.as<float>(), M, w.x.as<__nv_bfloat16>());
+    MLP_CUDA(cudaMemcpyAsync(w.xf, X, sizeof(float) * (size_t)M * ml::IN, cudaMemcpyHostToDevice, ss.s));
+    MLP_CUDA(cudaMemcpyAsync(w.params, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, ss.s));
+    ml::k_features_bf16<<<(M * ml::IN_PAD + 255) / 256, 256, 0, ss.s>>>(w.xf, M, w.x);
     rc = mlp_pack(w, ss.s);
     if (rc) return rc;
-    ml::k_forward<<<mlp_blocks(M), 128, ml::FWD_SMEM, ss.s>>>(w.x.as<__nv_bfloat16>(), M, w.wpack.as<__nv_bfloat16>(),
-                                                            w.params.as<float>(), w.y.as<float>(), nullptr);
+    ml::k_forward<<<mlp_blocks(M), 128, ml::FWD_SMEM, ss.s>>>(w.x, M, w.wpack, w.params, w.y, nullptr);
     MLP_CUDA(cudaGetLastError());
-    MLP_CUDA(cudaMemcpyAsync(y, w.y.p, sizeof(float) * M, cudaMemcpyDeviceToHost, ss.s));
+    MLP_CUDA(cudaMemcpyAsync(y, w.y, sizeof(float) * M, cudaMemcpyDeviceToHost, ss.s));
     MLP_CUDA(cudaStreamSynchronize(ss.s));
     return BTE_OK;
 }
@@ -3430,19 +3456,19 @@ bte_status bte_mlp_gradient(const float* X, const float* Y, int M, const float* 
     ScopedStream ss;
     MLP_CUDA(cudaStreamCreateWithFlags(&ss.s, cudaStreamNonBlocking));
     MlpWork w;
-    bte_status rc = mlp_alloc(w, M);
+    w.arrays(M, true);
+    w.slab.add(w.xf, (size_t)M * ml::IN);
+    bte_status rc = w.alloc();
     if (rc) return rc;
-    DevBuf xf;
-    MLP_CUDA(xf.alloc(sizeof(float) * (size_t)M * ml::IN));
-    MLP_CUDA(cudaMemcpyAsync(xf.p, X, sizeof(float) * (size_t)M * ml::IN, cudaMemcpyHostToDevice, ss.s));
-    MLP_CUDA(cudaMemcpyAsync(w.t.p, Y, sizeof(float) * M, cudaMemcpyHostToDevice, ss.s));
-    MLP_CUDA(cudaMemcpyAsync(w.params.p, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, ss.s));
-    ml::k_features_bf16<<<(M * ml::IN_PAD + 255) / 256, 256, 0, ss.s>>>(xf.as<float>(), M, w.x.as<__nv_bfloat16>());
+    MLP_CUDA(cudaMemcpyAsync(w.xf, X, sizeof(float) * (size_t)M * ml::IN, cudaMemcpyHostToDevice, ss.s));
+    MLP_CUDA(cudaMemcpyAsync(w.t, Y, sizeof(float) * M, cudaMemcpyHostToDevice, ss.s));
+    MLP_CUDA(cudaMemcpyAsync(w.params, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, ss.s));
+    ml::k_features_bf16<<<(M * ml::IN_PAD + 255) / 256, 256, 0, ss.s>>>(w.xf, M, w.x);
     rc = mlp_pack(w, ss.s);
     if (rc) return rc;
     rc = mlp_loss_grad(w, M, ss.s, loss);
     if (rc) return rc;
-    MLP_CUDA(cudaMemcpyAsync(grad, w.grad.p, sizeof(float) * ml::NPARAM, cudaMemcpyDeviceToHost, ss.s));
+    MLP_CUDA(cudaMemcpyAsync(grad, w.grad, sizeof(float) * ml::NPARAM, cudaMemcpyDeviceToHost, ss.s));
     MLP_CUDA(cudaStreamSynchronize(ss.s));
     return BTE_OK;
 }
@@ -3457,21 +3483,24 @@ bte_status bte_mlp_train(const float* X, const float* Y, int M, int steps, int b
     MLP_CUDA(cudaStreamCreateWithFlags(&ss.s, cudaStreamNonBlocking));
     cudaStream_t st = ss.s;
     MlpWork w;
-    bte_status rc = mlp_alloc(w, batch);
+    bf* xall = nullptr;
+    float *yall = nullptr, *m = nullptr, *v = nullptr;
+    int* idx = nullptr;
+    w.arrays(batch, true);
+    w.slab.add(w.xf, (size_t)M * ml::IN);
+    w.slab.add(xall, (size_t)M * ml::IN_PAD);
+    w.slab.add(yall, M);
+    w.slab.add(idx, M);
+    w.slab.add(m, ml::NPARAM);
+    w.slab.add(v, ml::NPARAM);
+    bte_status rc = w.alloc();
     if (rc) return rc;
-    DevBuf xf;
-    MLP_CUDA(xf.alloc(sizeof(float) * (size_t)M * ml::IN));
-    MLP_CUDA(w.xall.alloc(sizeof(bf) * (size_t)M * ml::IN_PAD));
-    MLP_CUDA(w.yall.alloc(sizeof(float) * M));
-    MLP_CUDA(w.idx.alloc(sizeof(int) * M));
-    MLP_CUDA(w.m.alloc(sizeof(float) * ml::NPARAM));
-    MLP_CUDA(w.v.alloc(sizeof(float) * ml::NPARAM));
-    MLP_CUDA(cudaMemsetAsync(w.m.p, 0, sizeof(float) * ml::NPARAM, st));
-    MLP_CUDA(cudaMemsetAsync(w.v.p, 0, sizeof(float) * ml::NPARAM, st));
-    MLP_CUDA(cudaMemcpyAsync(xf.p, X, sizeof(float) * (size_t)M * ml::IN, cudaMemcpyHostToDevice, st));
-    MLP_CUDA(cudaMemcpyAsync(w.yall.p, Y, sizeof(float) * M, cudaMemcpyHostToDevice, st));
-    MLP_CUDA(cudaMemcpyAsync(w.params.p, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, st));
-    ml::k_features_bf16<<<(M * ml::IN_PAD + 255) / 256, 256, 0, st>>>(xf.as<float>(), M, w.xall.as<bf>());
+    MLP_CUDA(cudaMemsetAsync(m, 0, sizeof(float) * ml::NPARAM, st));
+    MLP_CUDA(cudaMemsetAsync(v, 0, sizeof(float) * ml::NPARAM, st));
+    MLP_CUDA(cudaMemcpyAsync(w.xf, X, sizeof(float) * (size_t)M * ml::IN, cudaMemcpyHostToDevice, st));
+    MLP_CUDA(cudaMemcpyAsync(yall, Y, sizeof(float) * M, cudaMemcpyHostToDevice, st));
+    MLP_CUDA(cudaMemcpyAsync(w.params, params, sizeof(float) * ml::NPARAM, cudaMemcpyHostToDevice, st));
+    ml::k_features_bf16<<<(M * ml::IN_PAD + 255) / 256, 256, 0, st>>>(w.xf, M, xall);
     MLP_CUDA(cudaGetLastError());
     std::mt19937 rng(seed);
     std::vector<int> perm(M);
@@ -3482,13 +3511,12 @@ bte_status bte_mlp_train(const float* X, const float* Y, int M, int steps, int b
     for (int step = 0; step < steps; ++step) {
         if (pos + batch > M) {
             std::shuffle(perm.begin(), perm.end(), rng);
-            MLP_CUDA(cudaMemcpyAsync(w.idx.p, perm.data(), sizeof(int) * M, cudaMemcpyHostToDevice, st));
+            MLP_CUDA(cudaMemcpyAsync(idx, perm.data(), sizeof(int) * M, cudaMemcpyHostToDevice, st));
             MLP_CUDA(cudaStreamSynchronize(st));  // perm is reshuffled on the host next time
             pos = 0;
         }
-        ml::k_gather<<<(batch * ml::IN_PAD + 255) / 256, 256, 0, st>>>(w.xall.as<bf>(), w.yall.as<float>(),
-                                                                       w.idx.as<int>() + pos, batch, w.x.as<bf>(),
-                                                                       w.t.as<float>());
+        ml::k_gather<<<(batch * ml::IN_PAD + 255) / 256, 256, 0, st>>>(xall, yall, idx + pos, batch, w.x,
+                                                                       w.t);
         pos += batch;
         rc = mlp_pack(w, st);
         if (rc) return rc;
@@ -3498,11 +3526,10 @@ bte_status bte_mlp_train(const float* X, const float* Y, int M, int steps, int b
         if (loss_hist) loss_hist[step] = (float)loss;
         c1 *= b1;
         c2 *= b2;
-        ml::k_adam<<<(ml::NPARAM + 255) / 256, 256, 0, st>>>(w.params.as<float>(), w.grad.as<float>(), w.m.as<float>(),
-                                                              w.v.as<float>(), lr, b1, b2, eps, 1.f - c1, 1.f - c2);
+        ml::k_adam<<<(ml::NPARAM + 255) / 256, 256, 0, st>>>(w.params, w.grad, m, v, lr, b1, b2, eps, 1.f - c1, 1.f - c2);
         MLP_CUDA(cudaGetLastError());
     }
-    MLP_CUDA(cudaMemcpyAsync(params, w.params.p, sizeof(float) * ml::NPARAM, cudaMemcpyDeviceToHost, st));
+    MLP_CUDA(cudaMemcpyAsync(params, w.params, sizeof(float) * ml::NPARAM, cudaMemcpyDeviceToHost, st));
     MLP_CUDA(cudaStreamSynchronize(st));
     return BTE_OK;
 }
