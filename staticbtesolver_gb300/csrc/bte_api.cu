@@ -1410,7 +1410,10 @@ static const void* cluster_kernel(int slots) {
     // CTAs per SM the registers are limited for: two in FP64 (as many full ones
     // fit in shared memory), three in FP32
     constexpr int minb = sizeof(T) == 8 ? 2 : 3;
-    if constexpr (std::is_same<Op, bte::CsrOp>::value) return (const void*)bte::k_bicg_cluster<Op, T, 0, minb>;
+    if constexpr (bte::cluster_csr<Op>)  // (one system: one CTA per SM)
+        return slots == 3 ? (const void*)bte::k_bicg_cluster<Op, T, 3, 1>
+               : slots == 4 ? (const void*)bte::k_bicg_cluster<Op, T, 4, 1>
+                            : (const void*)bte::k_bicg_cluster<Op, T, 8, 1>;
     else
         return slots == 2 ? (const void*)bte::k_bicg_cluster<Op, T, 2, minb>
                : slots == 3 ? (const void*)bte::k_bicg_cluster<Op, T, 3, minb>
@@ -1444,17 +1447,17 @@ static cudaLaunchConfig_t cluster_config(int S, int ctas, int len, int slots, bo
 // what the FP64 pipes gain).
 constexpr int kClusterSpread = 512;
 template <typename Op, typename T>
-static int cluster_len(int device, int S, int n, int slots) {
+static int cluster_len(int device, int S, int n, int slots, bool best = true, int spread = kClusterSpread) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
     // (with three or four slots in FP64, two CTAs share an SM up to 1,792 cells)
     const int cells = sizeof(T) == 8 && slots > 2 && n <= 1792 * bte::KC_CTAS ? 1792 : bte::KC_CELLS;
-    const int ctas = std::max((n + cells - 1) / cells, std::min({bte::KC_CTAS, sms / S, n / kClusterSpread}));
+    const int ctas = std::max((n + cells - 1) / cells, std::min({bte::KC_CTAS, sms / S, n / spread}));
     if (ctas > bte::KC_CTAS) return 0;
     const int len = ((n + ctas - 1) / ctas + 31) & ~31;
     const void* k = cluster_kernel<Op, T>(slots);
     cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = cluster_config<T>(S, (n + len - 1) / len, len, slots, true, nullptr, &attr);
+    const cudaLaunchConfig_t cfg = cluster_config<T>(S, (n + len - 1) / len, len, slots, best, nullptr, &attr);
     int clusters = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
@@ -1518,6 +1521,21 @@ static bte_status batch_len(bte_ctx* ctx, int S, int prec, int* len) {
     }
     *len = ctx->kc_len[prec];
     return BTE_OK;
+}
+
+// One CSR system whose rows have at most `most` entries: slots (0: the phase
+// kernels, for longer rows, more unknowns than a cluster holds, and under
+// BTE_KRYLOV=phase) and cells per CTA.  The other SMs are idle, so a system gets
+// a CTA for every 256 unknowns, up to a cluster's 16 (2,048 unknowns, 82 steps:
+// of 64, 128, 256, 512 and 1,024 each 775, 772, 745, 815, 965 us; 3,872: 1,048,
+// 1,059, 1,100, 1,136, 1,449 us).
+static int csr_slots(int device, int n, int most, int* len) {
+    const int slots = most <= 3 ? 3 : most <= 4 ? 4 : 8;
+    *len = 0;
+    const char* v = std::getenv("BTE_KRYLOV");
+    if (most > slots || (v && v[0] == 'p') || n > bte::KC_CELLS * bte::KC_CTAS) return 0;
+    *len = cluster_len<bte::CsrOp, double>(device, 1, n, slots, false, 256);
+    return *len > 0 ? slots : 0;
 }
 
 static bte_status solve_batch_plain(bte_ctx* ctx, int b0, int nbb, const bte_options& o, bte_report& rep) {
@@ -2983,8 +3001,10 @@ bte_status bte_bicgstab_csr(int n, const int* rowptr, const int* colind, const d
     if (n <= 0 || !rowptr || !colind || !val || !b || !x || nnz < 0 || maxit <= 0 || !(tol > 0))
         return BTE_ERR_INVALID_ARGUMENT;
     if (rowptr[0] != 0 || rowptr[n] != nnz) return BTE_ERR_INVALID_ARGUMENT;
+    int most = 0;
     for (int i = 0; i < n; ++i)
         if (rowptr[i + 1] < rowptr[i]) return BTE_ERR_INVALID_ARGUMENT;
+        else most = std::max(most, rowptr[i + 1] - rowptr[i]);
     for (int k = 0; k < nnz; ++k)
         if (colind[k] < 0 || colind[k] >= n) return BTE_ERR_INVALID_ARGUMENT;
     bte_ctx tmp;  // scratch holder for error text and buffers
@@ -2996,40 +3016,51 @@ bte_status bte_bicgstab_csr(int n, const int* rowptr, const int* colind, const d
     cudaStream_t st = tmp.stream;
     const size_t Np = (size_t)((n + bte::CH - 1) / bte::CH) * bte::CH;
     const int nchunk = (int)(Np / bte::CH);
-    DevBuf d_rp, d_ci, d_v, d_x;
-    BTE_CUDA(d_rp.alloc(sizeof(int) * (n + 1)));
-    BTE_CUDA(d_ci.alloc(sizeof(int) * std::max(nnz, 1)));
-    BTE_CUDA(d_v.alloc(sizeof(double) * std::max(nnz, 1)));
-    BTE_CUDA(d_x.alloc(sizeof(double) * Np));
-    for (DevBuf* w : {&tmp.w_r, &tmp.w_rw, &tmp.w_p, &tmp.w_ph, &tmp.w_q, &tmp.w_z, &tmp.w_t, &tmp.w_b, &tmp.w_invD})
-        BTE_CUDA(w->alloc(sizeof(double) * Np));
-    BTE_CUDA(tmp.s_done.alloc(sizeof(int)));
-    BTE_CUDA(tmp.s_iters.alloc(sizeof(int)));
-    BTE_CUDA(tmp.s_flagA.alloc(sizeof(int) * 2));
-    BTE_CUDA(tmp.s_flagB.alloc(sizeof(int) * 2));
-    BTE_CUDA(tmp.s_rho.alloc(sizeof(double) * 2));
-    BTE_CUDA(tmp.s_alpha.alloc(sizeof(double)));
-    BTE_CUDA(tmp.s_omega.alloc(sizeof(double)));
-    BTE_CUDA(tmp.s_nrmr.alloc(sizeof(double)));
-    BTE_CUDA(tmp.s_nrm0.alloc(sizeof(double)));
-    BTE_CUDA(tmp.s_part.alloc(sizeof(double) * 7 * nchunk));
-    BTE_CUDA(tmp.s_active.alloc(sizeof(int) * (maxit + 2)));
-    BTE_CUDA(cudaMemcpyAsync(d_rp.p, rowptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st));
-    if (nnz > 0) {
-        BTE_CUDA(cudaMemcpyAsync(d_ci.p, colind, sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
-        BTE_CUDA(cudaMemcpyAsync(d_v.p, val, sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
+    int len = 0;
+    const int slots = csr_slots(dev, n, most, &len);
+    // state: done, iters, flagA[2], flagB[2], active; scal: rho[2], alpha, omega, nrmr, nrm0
+    DevSlab slab;
+    int *d_rp = nullptr, *d_ci = nullptr, *state = nullptr;
+    double *d_v = nullptr, *d_x = nullptr, *d_b = nullptr, *vec[8], *scal = nullptr, *parts = nullptr;
+    slab.add(d_rp, (size_t)n + 1);
+    slab.add(d_ci, nnz);
+    slab.add(d_v, nnz);
+    slab.add(d_x, Np);
+    slab.add(d_b, Np);
+    slab.add(state, slots ? 2 : 6 + (size_t)maxit + 2);
+    if (!slots) {
+        for (double*& w : vec) slab.add(w, Np);
+        slab.add(scal, 6);
+        slab.add(parts, 7 * (size_t)nchunk);
     }
-    BTE_CUDA(cudaMemsetAsync(tmp.w_b.p, 0, sizeof(double) * Np, st));
-    BTE_CUDA(cudaMemcpyAsync(tmp.w_b.p, b, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-    BTE_CUDA(cudaMemsetAsync(tmp.s_active.p, 0, sizeof(int) * (maxit + 2), st));
-    bte::CsrOp op{d_rp.as<int>(), d_ci.as<int>(), d_v.as<double>(), d_x.as<double>(), n, Np};
-    bte::BicgState bs{tmp.s_done.as<int>(), tmp.s_iters.as<int>(), tmp.s_flagA.as<int>(), tmp.s_flagB.as<int>(),
-                      tmp.s_rho.as<double>(), tmp.s_alpha.as<double>(), tmp.s_omega.as<double>(),
-                      tmp.s_nrmr.as<double>(), tmp.s_nrm0.as<double>(), nullptr, tmp.s_part.as<double>(),
-                      tmp.s_active.as<int>(), 1, nchunk, tol, maxit};
-    bte::BicgVecs<double> v{tmp.w_r.as<double>(), tmp.w_rw.as<double>(), tmp.w_p.as<double>(),
-                            tmp.w_ph.as<double>(), tmp.w_q.as<double>(), tmp.w_z.as<double>(),
-                            tmp.w_t.as<double>(), tmp.w_b.as<double>(), tmp.w_invD.as<double>(), Np};
+    BTE_CUDA(slab.alloc());
+    BTE_CUDA(cudaMemcpyAsync(d_rp, rowptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st));
+    if (nnz > 0) {
+        BTE_CUDA(cudaMemcpyAsync(d_ci, colind, sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
+        BTE_CUDA(cudaMemcpyAsync(d_v, val, sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
+    }
+    BTE_CUDA(cudaMemcpyAsync(d_b, b, sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    bte::CsrOp op{d_rp, d_ci, d_v, d_x, n, Np};
+    auto results = [&]() -> bte_status {
+        int out[2] = {0, 0};  // done, iters
+        BTE_CUDA(cudaMemcpyAsync(x, d_x, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+        BTE_CUDA(cudaMemcpyAsync(out, state, sizeof(out), cudaMemcpyDeviceToHost, st));
+        BTE_CUDA(cudaStreamSynchronize(st));
+        if (iterations) *iterations = out[1];
+        if (converged) *converged = (out[0] == 1 || out[0] == 2) ? 1 : 0;
+        return BTE_OK;
+    };
+    if (slots) {
+        const bte::ClusterSolve cs{state, state + 1, nullptr, n, len, tol, maxit, 1, 0, 0};
+        BTE_CUDA(launch_cluster(op, (const double*)d_b, Np, 1, slots, cs, st));
+        BTE_LAUNCHED();
+        return results();
+    }
+    if (Np > (size_t)n) BTE_CUDA(cudaMemsetAsync(d_b + n, 0, sizeof(double) * (Np - n), st));
+    BTE_CUDA(cudaMemsetAsync(state, 0, sizeof(int) * (6 + (size_t)maxit + 2), st));
+    bte::BicgState bs{state, state + 1, state + 2, state + 4, scal, scal + 2, scal + 3, scal + 4, scal + 5, nullptr,
+                      parts, state + 6, 1, nchunk, tol, maxit};
+    bte::BicgVecs<double> v{vec[0], vec[1], vec[2], vec[3], vec[4], vec[5], vec[6], d_b, vec[7], Np};
     dim3 grid(nchunk, 1);
     bte::k_bicg_init<<<grid, bte::THREADS, 0, st>>>(op, v, bs);
     BTE_LAUNCHED();
@@ -3057,14 +3088,7 @@ bte_status bte_bicgstab_csr(int n, const int* rowptr, const int* colind, const d
         BTE_CUDA(cudaStreamSynchronize(st));
         if (tmp.h_done.back() == 0 || last > maxit || i > maxit + 1) break;
     }
-    int done = 0, its = 0;
-    BTE_CUDA(cudaMemcpyAsync(x, d_x.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    BTE_CUDA(cudaMemcpyAsync(&done, bs.done, sizeof(int), cudaMemcpyDeviceToHost, st));
-    BTE_CUDA(cudaMemcpyAsync(&its, bs.iters, sizeof(int), cudaMemcpyDeviceToHost, st));
-    BTE_CUDA(cudaStreamSynchronize(st));
-    if (iterations) *iterations = its;
-    if (converged) *converged = (done == 1 || done == 2) ? 1 : 0;
-    return BTE_OK;
+    return results();
 }
 
 static bte_status dsa_solve_impl(bte_ctx* ctx, int n, int F, const int* nb, const double* W, const double* b,
@@ -3161,7 +3185,7 @@ constexpr size_t kNoAllocNp = ((size_t)kNoAllocMaxN + bte::CH - 1) / bte::CH * b
 constexpr int kNoAllocChunks = (int)(kNoAllocNp / bte::CH);
 // doubles: 10 vectors of kNoAllocNp (r, r_hat, p, p_hat, q, z, t, b, 1/D, x),
 // 7 x kNoAllocChunks partials, 8 scalars; then ints (done, iters, flagA[2],
-// flagB[2], error flag, spare, active[kNoAllocMaxIt + 2]) packed two per double.
+// flagB[2], error flag, longest row, active[kNoAllocMaxIt + 2]) packed two per double.
 constexpr size_t kNoAllocDoubles = 10 * kNoAllocNp + 7 * (size_t)kNoAllocChunks + 8;
 constexpr size_t kNoAllocInts = 8 + (size_t)kNoAllocMaxIt + 2;
 constexpr size_t kNoAllocScratch = kNoAllocDoubles + (kNoAllocInts + 1) / 2;
@@ -3172,12 +3196,16 @@ static_assert(kNoAllocScratchBytes < (size_t)24 << 20, "the static scratch is do
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratch];
 
 // Checks a caller's device CSR (row pointers non-decreasing from 0 to nnz,
-// column indices in range) before any kernel dereferences it.
+// column indices in range) before any kernel dereferences it, and finds the
+// length of its longest row.
 __global__ void k_noalloc_check_csr(const int* __restrict__ rowptr, const int* __restrict__ col, int n, int nnz,
-                                    int* bad) {
+                                    int* bad, int* most) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0 && (rowptr[0] != 0 || rowptr[n] != nnz)) atomicOr(bad, 1);
+    const int row = t < n ? rowptr[t + 1] - rowptr[t] : 0;
     if (t < n && rowptr[t + 1] < rowptr[t]) atomicOr(bad, 1);
+    const int longest = __reduce_max_sync(0xffffffffu, row);
+    if ((threadIdx.x & 31) == 0) atomicMax(most, longest);
     for (int k = t; k < nnz; k += gridDim.x * blockDim.x)
         if (col[k] < 0 || col[k] >= n) atomicOr(bad, 1);
 }
@@ -3242,41 +3270,48 @@ extern "C" bte_status bte_bicgstab_csr_noalloc(int n, const int* rowptr, const i
     launched = true;
     NOALLOC_CUDA(cudaMemsetAsync(iv, 0, sizeof(int) * (8 + (size_t)maxit + 2), st));
     NOALLOC_CUDA(cudaMemsetAsync(vec[7], 0, sizeof(double) * Np, st));
-    k_noalloc_check_csr<<<(n + 255) / 256, 256, 0, st>>>(rowptr, colind, n, nnz, bad);
+    k_noalloc_check_csr<<<(n + 255) / 256, 256, 0, st>>>(rowptr, colind, n, nnz, bad, bad + 1);
     NOALLOC_CUDA(cudaGetLastError());
-    int h_bad = 0;
-    NOALLOC_CUDA(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int h_bad[2] = {0, 0};
+    NOALLOC_CUDA(cudaMemcpyAsync(h_bad, bad, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     NOALLOC_CUDA(cudaStreamSynchronize(st));
-    if (h_bad) {
+    if (h_bad[0]) {
         g_create_error = "bte_bicgstab_csr_noalloc: malformed CSR (row pointers or column indices)";
         return BTE_ERR_INVALID_ARGUMENT;
     }
     NOALLOC_CUDA(cudaMemcpyAsync(vec[7], b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
     bte::CsrOp op{rowptr, colind, val, vec[9], n, Np};
-    bte::BicgState bs{done, iters, flagA, flagB, sc, sc + 2, sc + 3, sc + 4, sc + 5, nullptr, part, active, 1, nchunk,
-                      tol, maxit};
-    bte::BicgVecs<double> v{vec[0], vec[1], vec[2], vec[3], vec[4], vec[5], vec[6], vec[7], vec[8], Np};
-    dim3 grid(nchunk, 1);
-    bte::k_bicg_init<<<grid, bte::THREADS, 0, st>>>(op, v, bs);
-    bte::k_bicg_init_scalars<<<1, 32, 0, st>>>(bs, nullptr);
-    NOALLOC_CUDA(cudaGetLastError());
-    int i = 1;
-    for (;;) {
-        int last = i;
-        for (int g = 0; g < kGroup && i <= maxit + 1; ++g, ++i) {
-            bte::k_bicg_p<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
-            last = i;
-            if (i > maxit) break;
-            bte::k_bicg_spmv1<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
-            bte::k_bicg_s<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
-            bte::k_bicg_spmv2<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
-            bte::k_bicg_x<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
-        }
+    int dev = 0, len = 0;
+    NOALLOC_CUDA(cudaGetDevice(&dev));
+    if (const int slots = csr_slots(dev, n, h_bad[1], &len)) {
+        const bte::ClusterSolve cs{done, iters, nullptr, n, len, tol, maxit, 1, 0, 0};
+        NOALLOC_CUDA(launch_cluster(op, (const double*)vec[7], Np, 1, slots, cs, st));
+    } else {
+        bte::BicgState bs{done, iters, flagA, flagB, sc, sc + 2, sc + 3, sc + 4, sc + 5, nullptr, part, active, 1,
+                          nchunk, tol, maxit};
+        bte::BicgVecs<double> v{vec[0], vec[1], vec[2], vec[3], vec[4], vec[5], vec[6], vec[7], vec[8], Np};
+        dim3 grid(nchunk, 1);
+        bte::k_bicg_init<<<grid, bte::THREADS, 0, st>>>(op, v, bs);
+        bte::k_bicg_init_scalars<<<1, 32, 0, st>>>(bs, nullptr);
         NOALLOC_CUDA(cudaGetLastError());
-        int h_active = 0;
-        NOALLOC_CUDA(cudaMemcpyAsync(&h_active, active + last, sizeof(int), cudaMemcpyDeviceToHost, st));
-        NOALLOC_CUDA(cudaStreamSynchronize(st));
-        if (h_active == 0 || last > maxit || i > maxit + 1) break;
+        int i = 1;
+        for (;;) {
+            int last = i;
+            for (int g = 0; g < kGroup && i <= maxit + 1; ++g, ++i) {
+                bte::k_bicg_p<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
+                last = i;
+                if (i > maxit) break;
+                bte::k_bicg_spmv1<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
+                bte::k_bicg_s<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
+                bte::k_bicg_spmv2<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
+                bte::k_bicg_x<<<grid, bte::THREADS, 0, st>>>(op, v, bs, i);
+            }
+            NOALLOC_CUDA(cudaGetLastError());
+            int h_active = 0;
+            NOALLOC_CUDA(cudaMemcpyAsync(&h_active, active + last, sizeof(int), cudaMemcpyDeviceToHost, st));
+            NOALLOC_CUDA(cudaStreamSynchronize(st));
+            if (h_active == 0 || last > maxit || i > maxit + 1) break;
+        }
     }
     NOALLOC_CUDA(cudaMemcpyAsync(x, vec[9], sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
     int h_state[2] = {0, 0};

@@ -28,7 +28,10 @@
 // Solves measured, phase kernels -> clusters: 578 triangles x 32 directions to
 // margin 1e-5, 135 -> 17.4 ms; 750 tetrahedra x 128 directions, 228 -> 43 ms;
 // 20,000 triangles x 256 systems, two outer iterations, 199 -> 84 ms; 10,082
-// triangles x 256 systems in mixed precision, three, 157 -> 25 ms.
+// triangles x 256 systems in mixed precision, three, 157 -> 25 ms.  One CSR
+// system from host arrays, to 1e-12: 968 unknowns 2.8 -> 0.56 ms, 9,800 unknowns
+// 10.0 -> 1.9 ms (9 us a step: 3.7 of the FP64 pipe, the rest barriers and remote
+// loads), 32,768 unknowns 20.5 -> 5.6 ms.
 // Sums are taken in a fixed order (threads, warps, CTAs), so a solve is
 // reproducible to the bit; they are grouped differently from the phase
 // kernels', so the two agree to rounding.
@@ -91,7 +94,7 @@ __device__ __forceinline__ void cluster_load(unsigned a, float& v) {
 
 // Dynamic shared memory of k_bicg_cluster for len cells per CTA: the exchanged
 // vector, x, r_hat, (best iterate); SLOTS coefficients and neighbour places
-// per cell, or 1/D for a CSR operator (slots = 0).
+// per cell.
 template <typename T>
 __host__ __device__ constexpr int cluster_row_group() { return sizeof(T) == 4 ? 4 : 1; }
 template <typename T>
@@ -102,13 +105,18 @@ __host__ __device__ constexpr int cluster_cells(int len) {
 template <typename T>
 constexpr size_t cluster_smem_bytes(int len, int slots, bool best) {
     const size_t cells = cluster_cells<T>(len);
-    return cells * (sizeof(T) * (3 + (best ? 1 : 0) + (slots ? slots : 1)) + sizeof(uint32_t) * slots);
+    return cells * (sizeof(T) * (3 + (best ? 1 : 0) + slots) + sizeof(uint32_t) * slots);
 }
 
 // One system per cluster (y = blockIdx.x / CTAs of the cluster) of
 // ceil(n / len) CTAs, len <= KC_CELLS a multiple of 32.  rhs: [S][Np]; the solution goes to op.x_of(y), the outcome to
-// done and iters.  SLOTS >= the largest number of nonzero fc of a cell, or 0
-// for a CSR operator.  MINB: CTAs per SM the registers are limited for.
+// done and iters.  SLOTS >= the largest number of nonzero fc of a cell, or of
+// entries of a row for a CSR operator.  MINB: CTAs per SM the registers are
+// limited for.
+template <typename Op>
+constexpr bool cluster_csr = false;
+template <>
+inline constexpr bool cluster_csr<CsrOp> = true;
 #define BTE_CLUSTER_ROWS(k)                                        \
     _Pragma("unroll") for (int _g = 0; _g < KC_ROWS / G && _g < groups; ++_g) \
         _Pragma("unroll") for (int _r = 0, k = _g * G; _r < G; ++_r, ++k)
@@ -132,12 +140,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_bicg_cluster(Op op, const T* 
     const int mine = max(0, min(st.len, st.n - first));
     const int cells = cluster_cells<T>(st.len);                    // slots of the arrays below
     const bool lead = rank == 0 && tid == 0;
-    T* sv = reinterpret_cast<T*>(kc_smem);  // the exchanged vector: p, then s (CSR: M p, M s)
+    T* sv = reinterpret_cast<T*>(kc_smem);  // the exchanged vector: p, then s
     T* sx = sv + cells;                     // M^-1 x
     T* srw = sx + cells;
     T* sxb = srw + cells;                   // with st.best
-    T* scf = sxb + (st.best ? cells : 0);   // [row][SLOTS][THREADS] coefficients (CSR: 1/D)
-    uint32_t* sat = reinterpret_cast<uint32_t*>(scf + (size_t)(SLOTS ? SLOTS : 1) * cells);  // ... the neighbours' places
+    T* scf = sxb + (st.best ? cells : 0);   // [row][SLOTS][THREADS] coefficients of A M
+    uint32_t* sat = reinterpret_cast<uint32_t*>(scf + (size_t)SLOTS * cells);  // ... the neighbours' places
     T* xout = op.x_of(y);
     // a warp's rows of 32 cells are taken in groups of G, without a branch
     // inside a group so their loads overlap: the ones with a cell in it.  FP64
@@ -208,27 +216,14 @@ __global__ void __launch_bounds__(THREADS, MINB) k_bicg_cluster(Op op, const T* 
         a = __shfl_sync(0xffffffffu, s, 0);
         b = __shfl_sync(0xffffffffu, s, 16);
     };
-    // (A M v)[c] of row k, v exchanged
+    // (A M v)[c] of row k, v exchanged (face flux: the diagonal of A M is 1)
     auto product = [&](int k, T v) {
-        if constexpr (SLOTS > 0) {
-            T x[SLOTS], s = v;
+        T x[SLOTS], s = cluster_csr<Op> ? (T)0 : v;
 #pragma unroll
-            for (int f = 0; f < SLOTS; ++f) cluster_load(sat[(k * SLOTS + f) * THREADS + tid], x[f]);
+        for (int f = 0; f < SLOTS; ++f) cluster_load(sat[(k * SLOTS + f) * THREADS + tid], x[f]);
 #pragma unroll
-            for (int f = 0; f < SLOTS; ++f) s = fmat(scf[(k * SLOTS + f) * THREADS + tid], x[f], s);
-            return s;
-        } else {
-            const int l = k * THREADS + tid, c = first + l;
-            T s = 0;
-            if (l >= mine) return s;
-            const int k1 = op.rowptr[c + 1];
-            for (int e = op.rowptr[c]; e < k1; ++e) {
-                T x;
-                cluster_load(place(op.col[e]), x);
-                s = fmat((T)op.val[e], x, s);
-            }
-            return s;
-        }
+        for (int f = 0; f < SLOTS; ++f) s = fmat(scf[(k * SLOTS + f) * THREADS + tid], x[f], s);
+        return s;
     };
 
     T r[KC_ROWS], p[KC_ROWS], q[KC_ROWS], t[KC_ROWS];
@@ -237,12 +232,28 @@ __global__ void __launch_bounds__(THREADS, MINB) k_bicg_cluster(Op op, const T* 
         // 1/D of every cell, exchanged once to scale the coefficients
         BTE_CLUSTER_ROWS(k) {
             const int l = k * THREADS + tid;
-            const T d = l < mine ? (T)op.inv_diag(y, first + l) : (T)0;
-            if constexpr (SLOTS > 0) sv[l] = d;
-            else scf[l] = d;
+            sv[l] = l < mine ? (T)op.inv_diag(y, first + l) : (T)0;
         }
         cluster_barrier(ctas);
-        if constexpr (SLOTS > 0) {
+        // (two loops: sharing one costs the FP32 kernel 3 % by its registers)
+        if constexpr (cluster_csr<Op>) {
+            BTE_CLUSTER_ROWS(k) {
+                const int l = k * THREADS + tid, c = first + l;
+                int m = 0;
+                if (l < mine)
+                    for (int e = op.rowptr[c]; e < op.rowptr[c + 1] && m < SLOTS; ++e, ++m) {
+                        const unsigned at = place(op.col[e]);
+                        T d;
+                        cluster_load(at, d);
+                        scf[(k * SLOTS + m) * THREADS + tid] = (T)op.val[e] * d;
+                        sat[(k * SLOTS + m) * THREADS + tid] = at;
+                    }
+                for (; m < SLOTS; ++m) {
+                    scf[(k * SLOTS + m) * THREADS + tid] = 0;
+                    sat[(k * SLOTS + m) * THREADS + tid] = cluster_map(sv_a + (unsigned)sizeof(T) * (unsigned)l, rank);
+                }
+            }
+        } else {
             int sb, sd;
             op.bd(y, sb, sd);
             const T kb = op.kb[sb];
@@ -378,7 +389,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_bicg_cluster(Op op, const T* 
 #pragma unroll
             for (int k = 0; k < KC_ROWS; ++k) {
                 const int l = k * THREADS + tid;
-                if (l < mine) xout[first + l] = (SLOTS > 0 ? (T)op.inv_diag(y, first + l) : scf[l]) * xs[l];
+                if (l < mine) xout[first + l] = (T)op.inv_diag(y, first + l) * xs[l];
             }
             // the padding cells of the system stay zero
             for (int c = st.n + (int)rank * THREADS + tid; c < (int)Np; c += (int)ctas * THREADS) xout[c] = 0;
@@ -397,7 +408,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_bicg_cluster(Op op, const T* 
                 T u = fmat(-om, q[k], p[k]);
                 u = fmat(bt, u, r[k]);
                 p[k] = u;
-                sv[l] = SLOTS > 0 ? u : scf[l] * u;
+                sv[l] = u;
             }
         }
         cluster_barrier(ctas);
@@ -434,7 +445,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_bicg_cluster(Op op, const T* 
             const int l = k * THREADS + tid;
             const T s = fmat(-al, q[k], r[k]);
             r[k] = s;
-            sv[l] = SLOTS > 0 ? s : scf[l] * s;
+            sv[l] = s;
         }
         cluster_barrier(ctas);
         {  // t = A M s, t . s, t . t
