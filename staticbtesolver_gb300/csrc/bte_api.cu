@@ -1341,8 +1341,7 @@ static bte_status level_plan(bte_ctx* ctx) {
     bte::SweepPlan sp{ctx->p_cell.as<int>(), ctx->p_bidx.as<int>(), ctx->p_dg.as<double>(), ctx->p_vo.as<double>(),
                       ctx->p_nb.as<int>(), ctx->p_fc.as<double>(), ctx->p_lvl.as<int>(), ctx->p_lvl_off.as<int>(), n, F,
                       ctx->n2};
-    bte::k_sweep_invd<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(sp, ctx->d_kb.as<double>(), ctx->d_Cb.as<double>(),
-                                                                 ctx->solid_angle, ctx->n_band, ND,
+    bte::k_sweep_invd<<<dim3((n + 255) / 256, ND), 256, 0, st>>>(sp, ctx->d_kb.as<double>(), ctx->n_band, ND,
                                                                  ctx->p_voi.as<double>(), ctx->p_kinv.as<double>());
     BTE_LAUNCHED();
     ctx->level_ready = true;
@@ -1369,9 +1368,8 @@ static bte_status stream_plan(bte_ctx* ctx) {
     BTE_CUDA(ctx->st_voi.alloc(sizeof(double) * ctx->n_band * ND * npad));
     BTE_CUDA(ctx->st_kinv.alloc(sizeof(double) * ctx->n_band * ND * npad));
     bte::k_stream_invd<<<dim3((unsigned)((npad + 255) / 256), ND), 256, 0, st>>>(
-        ctx->st_cell.as<int>(), ctx->d_dg.as<double>(), ctx->d_vo.as<double>(), ctx->d_kb.as<double>(),
-        ctx->d_Cb.as<double>(), ctx->solid_angle, ctx->n_band, ND, ctx->Np, npad, ctx->st_voi.as<double>(),
-        ctx->st_kinv.as<double>());
+        ctx->st_cell.as<int>(), ctx->d_dg.as<double>(), ctx->d_vo.as<double>(), ctx->d_kb.as<double>(), ctx->n_band, ND,
+        ctx->Np, npad, ctx->st_voi.as<double>(), ctx->st_kinv.as<double>());
     BTE_LAUNCHED();
     ctx->stream_ready = true;
     return BTE_OK;
@@ -2170,7 +2168,8 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
                        src, ctx->d_bcell.as<int>(), ctx->nbcell, ctx->d_kb.as<double>(), ctx->p_binvd.as<double>(),
                        nbb, b0, ctx->d_bsum.as<double>()));
     }
-    const bte::SweepSrc ssrc{ctx->d_T.as<double>(), ctx->T_ref, ctx->d_bsum.as<double>(), ctx->e_prev, ctx->nbcell};
+    const bte::SweepSrc ssrc{ctx->d_ebar.as<double>(), ctx->d_T.as<double>(), ctx->d_Cb.as<double>(), ctx->T_ref,
+                             ctx->solid_angle, ctx->d_bsum.as<double>(), ctx->e_prev, ctx->nbcell};
     // launch-shape autotuning on the first sweep of this plan (each candidate
     // computes the same x from the same inputs); the choice is kept per
     // process for the same device and plan shape, so a new context on the

@@ -18,8 +18,8 @@
 //    band k/D and V Omega/D -- into NCH buffers (cp.async.bulk, completion on
 //    an mbarrier), NCH chunks ahead at most;
 //  * H helpers turn the chunks' V Omega/D into right-hand sides in place
-//    (theta V Omega/D + boundary part / D, theta = T - T_ref gathered once per
-//    block, not per band), and fetch the upstream values that are too old for
+//    (ebar V Omega/D + boundary part / D, ebar = C_b / Omega_tot (T - T_ref) with
+//    T gathered once per block, not ebar per band), and fetch the upstream values that are too old for
 //    the ring into the chunk's annex of it;
 //  * WC consumer warps per band solve the levels, with a barrier among
 //    themselves only: the bands of a block drift apart by up to NCH chunks, so
@@ -125,12 +125,11 @@ __global__ void k_stream_order(const int* __restrict__ lo_perm, const uint8_t* _
 }
 
 // The diagonal folded into the sweep's coefficients per band and padded
-// position, as k_sweep_invd: voi = C_b / Omega_tot vo / D, kinv = k_b / D (0
+// position, as k_sweep_invd: voi = vo / D, kinv = k_b / D (0
 // where there is no cell).
 __global__ void k_stream_invd(const int* __restrict__ cell, const double* __restrict__ dg,
-                              const double* __restrict__ vo, const double* __restrict__ kb,
-                              const double* __restrict__ Cb, double solid_angle, int n_band, int n_dir, size_t Np,
-                              size_t npad, double* __restrict__ voi, double* __restrict__ kinv) {
+                              const double* __restrict__ vo, const double* __restrict__ kb, int n_band, int n_dir,
+                              size_t Np, size_t npad, double* __restrict__ voi, double* __restrict__ kinv) {
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int d = blockIdx.y;
     if (p >= npad) return;
@@ -139,7 +138,7 @@ __global__ void k_stream_invd(const int* __restrict__ cell, const double* __rest
     for (int b = 0; b < n_band; ++b) {
         const size_t q = ((size_t)b * n_dir + d) * npad + p;
         const double invD = c >= 0 ? 1.0 / fma(kb[b], g, v) : 0.0;
-        voi[q] = Cb[b] / solid_angle * (v * invD);
+        voi[q] = v * invD;
         kinv[q] = kb[b] * invD;
     }
 }
@@ -366,6 +365,7 @@ __global__ void __launch_bounds__(STHREADS, 1) k_sweep_stream(StreamPlan sp, Str
         const unsigned* fd = sp.far + (size_t)d * sp.nq * (FM * SCH);
         const size_t row = ((size_t)(b0 + g0) * n_dir + d) * Np, band = (size_t)n_dir * Np;
         constexpr int R = SCH / 32;
+        const double cs = lane < gn ? src.Cb[b0 + g0 + lane] / src.solid_angle : 0.0;  // band g's in lane g
         int m = h < nq ? nf[h] : 0, m2 = h + sh.H < nq ? nf[h + sh.H] : 0;
         unsigned e[R];
 #pragma unroll
@@ -413,6 +413,7 @@ __global__ void __launch_bounds__(STHREADS, 1) k_sweep_stream(StreamPlan sp, Str
 #pragma unroll
             for (int r = 0; r < R; ++r) T[r] -= src.T_ref;
             for (int g = 0; g < gn; ++g) {
+                const double cg = __shfl_sync(0xffffffffu, cs, g);
                 double bs[R] = {};
                 if (wall) {
                     const double* bb = src.bsum + ((size_t)d * nbb + g0 + g) * src.nbcell;
@@ -423,7 +424,7 @@ __global__ void __launch_bounds__(STHREADS, 1) k_sweep_stream(StreamPlan sp, Str
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     double* v = kv + (size_t)(2 * g + 1) * span + r * 32;
-                    *v = fma(T[r], *v, bs[r]);
+                    *v = fma(cg * T[r], *v, bs[r]);
                 }
             }
             fence_proxy_async_smem();

@@ -319,14 +319,12 @@ struct SweepPlan {
 
 // The diagonal folded into the sweep's coefficients, per system in level
 // order: with D = k_b dg[d][j] + vo[d][j],
-//   voi[b][d][j] = C_b / Omega_tot vo / D,   kinv[b][d][j] = k_b / D,
-// so x = (R - k_b off) / D becomes x = theta voi + bs/D - kinv off with theta =
-// T - T_ref, the same for every band: two FP64 operations per cell fewer in the
-// sweep (GB300 issues FP64 at ~2 lanes per SM per clock) and one gather for all
-// bands of a block.  The diagonal does not change across outer iterations: once
-// per solve.
-__global__ void k_sweep_invd(SweepPlan sp, const double* __restrict__ kb, const double* __restrict__ Cb,
-                             double solid_angle, int n_band, int n_dir, double* voi, double* kinv) {
+//   voi[b][d][j] = vo / D,   kinv[b][d][j] = k_b / D,
+// so x = (R - k_b off) / D becomes x = ebar voi + bs/D - kinv off: two FP64
+// operations per cell fewer in the sweep (GB300 issues FP64 at ~2 lanes per SM
+// per clock).  The diagonal does not change across outer iterations: once per solve.
+__global__ void k_sweep_invd(SweepPlan sp, const double* __restrict__ kb, int n_band, int n_dir, double* voi,
+                             double* kinv) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int d = blockIdx.y;
     if (j >= sp.n) return;
@@ -335,7 +333,7 @@ __global__ void k_sweep_invd(SweepPlan sp, const double* __restrict__ kb, const 
     for (int b = 0; b < n_band; ++b) {
         const double invD = 1.0 / fma(kb[b], dg, vo);
         const size_t q = ((size_t)b * n_dir + d) * sp.n2 + j;
-        voi[q] = Cb[b] / solid_angle * (vo * invD);
+        voi[q] = vo * invD;
         kinv[q] = kb[b] * invD;
     }
 }
@@ -350,12 +348,14 @@ struct SweepItem {
     double kinv, voi, eb, bs, old;
 };
 
-// The cell-addressed operands come from SweepSrc (the temperature of the
-// source, the boundary part of the right-hand side, and with MARGIN the
-// previous iterate).
+// The cell-addressed operands come from SweepSrc (ebar, the boundary part of
+// the right-hand side, and with MARGIN the previous iterate; T and C_b for
+// k_sweep_stream, which forms ebar).
 struct SweepSrc {
+    const double* ebar;   // [n_band][Np]
     const double* T;      // [Np]
-    double T_ref;
+    const double* Cb;     // [n_band]
+    double T_ref, solid_angle;
     const double* bsum;   // [nbb * n_dir][nbcell] (k_bound_rhs)
     const double* x_old;  // e_prev
     int nbcell;
@@ -370,8 +370,7 @@ struct SweepRows {
     const double* fc;  // [F][n]
     const double* voi; // [n] this band
     const double* kinv;
-    const double* T;   // source temperature, by cell
-    double T_ref;
+    const double* eb;  // ebar of this band, by cell
     const double* bs;  // boundary part of this system, by boundary row
     const double* xold;
     int n, F;
@@ -395,7 +394,7 @@ __device__ __forceinline__ void sweep_load_a(const SweepRows& r, int j, SweepIte
 // cell index has arrived and the loads do not stall the sweep.
 template <bool MARGIN, int FM>
 __device__ __forceinline__ void sweep_load_b(const SweepRows& r, SweepItem<FM>& it) {
-    it.eb = r.T[it.c] - r.T_ref;
+    it.eb = r.eb[it.c];
     it.bs = it.bi >= 0 ? r.bs[it.bi] : 0.0;
     if (MARGIN) it.old = r.xold[it.c];
 }
@@ -458,8 +457,7 @@ __global__ void __launch_bounds__(128, 5) k_sweep(SweepPlan sp, const double* __
     rows.fc = sp.fc + (size_t)d * sp.F * n;
     rows.voi = voi + sys * sp.n2;
     rows.kinv = kinv + sys * sp.n2;
-    rows.T = src.T;
-    rows.T_ref = src.T_ref;
+    rows.eb = src.ebar + (size_t)b * Np;
     rows.bs = src.bsum + ((size_t)d * nbb + (b - b0)) * src.nbcell;
     rows.xold = src.x_old + sys * Np;
     rows.n = n;
@@ -660,8 +658,8 @@ __host__ __device__ constexpr size_t staged_smem_bytes(int cap, int G, int W) {
 // .. + G - 1 (thread t serves band t mod gp, positions t / gp, t / gp +
 // blockDim / gp, ... of each stage, as in k_sweep; cap = 2 blockDim / gp, so a
 // thread has at most two items per stage).  x = e_curr, x_old = e_prev
-// ([band][n_dir][Np]); kinv and voi [band][n_dir][n2] (all bands); src: the
-// source temperature and the boundary parts.  The ring keeps the last W solved positions per
+// ([band][n_dir][Np]); kinv and voi [band][n_dir][n2] (all bands); src: ebar
+// and the boundary parts.  The ring keeps the last W solved positions per
 // band: a position p is still there during the stage [j0, j1) whenever
 // p >= j1 - W.  A stage's copies that have not landed after kStagePolls polls
 // set *err; the block then waits (bounded) for its copies in flight and
@@ -694,6 +692,7 @@ __global__ void __launch_bounds__(256) k_sweep_staged(StagedPlan sp, const doubl
     const int n = sp.n, n2 = sp.n2;
     double* xb = x + ((size_t)(b0 + bb) * n_dir + d) * Np;
     const double* xo = x_old + ((size_t)(b0 + bb) * n_dir + d) * Np;
+    const double* eb = src.ebar + (size_t)(b0 + bb) * Np;
     const double* bsb = src.bsum + ((size_t)d * nbb + bb) * src.nbcell;
     double* rg = ring + (size_t)bl * W;
     const int* cell_d = sp.cell + (size_t)d * n;
@@ -740,7 +739,7 @@ __global__ void __launch_bounds__(256) k_sweep_staged(StagedPlan sp, const doubl
             const int j = j0 + tpos + k * per_round;
             if (j >= j1) continue;
             const int2 cb = *reinterpret_cast<const int2*>(B + (size_t)(j - j0) * L::bytes);
-            geb[k] = src.T[cb.x] - src.T_ref;
+            geb[k] = eb[cb.x];
             gbs[k] = cb.y >= 0 ? bsb[cb.y] : 0.0;
         }
     };
