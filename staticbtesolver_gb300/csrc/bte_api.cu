@@ -147,7 +147,7 @@ struct bte_ctx {
     DevBuf d_dg, d_vo, d_fc, d_nb, d_kb, d_Cb, d_Lr, d_vg;
     DevBuf d_bptr, d_bf_cell, d_bf_kind, d_bf_bc, d_bf_diff, d_cin, d_eiso, d_mirror, d_ediff;
     DevBuf d_dlist, d_wdiff, d_wden, d_hw, d_bf_area;
-    DevBuf d_e0, d_e1, d_ebar, d_Tb, d_T, d_mpart, d_margin, d_hpart, d_qband, d_q;
+    DevBuf d_e0, d_e1, d_ebar, d_Tb, d_T, d_mpart, d_count, d_hpart, d_qband, d_q;
     // batch work
     int nbb = 0;
     DevBuf w_r, w_rw, w_p, w_ph, w_q, w_z, w_t, w_b, w_invD, w_xb;
@@ -676,8 +676,8 @@ static bte_status setup(bte_ctx* ctx, int batch_systems) {
     BTE_CUDA(ctx->d_ebar.alloc(sizeof(double) * NB * Np));
     BTE_CUDA(ctx->d_Tb.alloc(sizeof(double) * NB * Np));
     BTE_CUDA(ctx->d_T.alloc(sizeof(double) * Np));
-    BTE_CUDA(ctx->d_mpart.alloc(sizeof(double) * NB * (Np / bte::THREADS + 1)));
-    BTE_CUDA(ctx->d_margin.alloc(sizeof(double) * 2));
+    BTE_CUDA(ctx->d_mpart.alloc(sizeof(double) * std::max((size_t)bte::reduce_groups(ctx->n), NB * (Np / bte::THREADS + 1))));
+    BTE_CUDA(ctx->d_count.alloc(sizeof(unsigned)));
     BTE_CUDA(ctx->d_hpart.alloc(sizeof(double) * NB * std::max(nbf, 1)));
     BTE_CUDA(ctx->d_qband.alloc(sizeof(double) * std::max(ctx->n_bc, 1) * NB));
     BTE_CUDA(ctx->d_q.alloc(sizeof(double) * std::max(ctx->n_bc, 1)));
@@ -2536,6 +2536,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
     const bool post_step = o.accel != 0 || dsa_on;  // kernels after the margin read-back
     bte_status result = BTE_ERR_NOT_CONVERGED;
     const int nred = (int)(Np / bte::THREADS);
+    BTE_CUDA(cudaMemsetAsync(ctx->d_count.p, 0, sizeof(unsigned), st));
     // the sweep of an acyclic plan may sum the margin itself (k_reduce then
     // reads e_curr only); the choice is made with the launch shape, on the
     // first sweep, so it is read after the sweeps of an iteration
@@ -2630,7 +2631,8 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
                                ctx->e_prev, ctx->d_dlist.as<int>(), ctx->d_bf_cell.as<int>(), ctx->d_wdiff.as<double>(),
                                ctx->d_wden.as<double>(), ctx->ndiff, NB, ND, Np, ctx->nbf, ctx->d_ediff.as<double>()));
             }
-            if (acyclic_sweep) BTE_CUDA(cudaMemsetAsync(ctx->d_spart.p, 0, sizeof(double) * ND * NB, st));
+            if (acyclic_sweep && (it == 0 || fused_margin()))  // (whether the sweep sums it is chosen in the first one)
+                BTE_CUDA(cudaMemsetAsync(ctx->d_spart.p, 0, sizeof(double) * ND * NB, st));
             if (timed) BTE_CUDA(cudaEventRecord(ev[1], st));
             for (int b0 = 0; b0 < NB; b0 += ctx->nbb) {
                 const int nbb = std::min(ctx->nbb, NB - b0);
@@ -2641,6 +2643,19 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
             }
             if (timed) BTE_CUDA(cudaEventRecord(ev[2], st));
             const bool fused = fused_margin();
+            // (the margin goes straight to the host: nothing on the device reads it)
+            if (ctx->dim != 1 && bte::reduce_by_cells(ctx->n, NB, ND)) {  // (1D Krylov solves follow the last bit, see batch_len)
+                const bte::ReduceArgs ra{ctx->e_curr, ctx->e_prev, ctx->d_omega.as<double>(), ctx->d_Cb.as<double>(),
+                                         ctx->d_Lr.as<double>(), Lr_sum, ctx->T_ref, ctx->solid_angle, ctx->n, NB, ND,
+                                         Np, ctx->d_Tb.as<double>(), ctx->d_T.as<double>(), ctx->d_ebar.as<double>(),
+                                         ctx->d_mpart.as<double>(), ctx->d_spart.as<double>(), ND * NB,
+                                         ctx->d_count.as<unsigned>(), ctx->h_pinned};
+                const int groups = bte::reduce_groups(ctx->n);
+                BTE_LAUNCH(KK_REDUCE, -1, ((fused ? 1.0 : 2.0) * NB * ND + 2.0 * NB + 1) * ctx->n * 8.0, 0,
+                           fused ? bte::k_reduce_cells<false><<<groups, bte::THREADS, 0, st>>>(ra)
+                                 : bte::k_reduce_cells<true><<<groups, bte::THREADS, 0, st>>>(ra));
+                return BTE_OK;
+            }
             if (fused) {
                 BTE_LAUNCH(KK_REDUCE, -1, (1.0 * NB * ND + NB) * ctx->n * 8.0, 0,
                            bte::k_reduce<false><<<dim3(nred, NB), bte::THREADS, 0, st>>>(
@@ -2660,7 +2675,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
             // margin = sum of the partials / (n_band n_cell), fixed order
             bte::k_margin_final<<<1, bte::THREADS, 0, st>>>(fused ? ctx->d_spart.as<double>() : ctx->d_mpart.as<double>(),
                                                             fused ? ND * NB : nred * NB, (double)NB * ctx->n,
-                                                            ctx->d_margin.as<double>());
+                                                            ctx->h_pinned);
             BTE_LAUNCHED();
             return BTE_OK;
         };
@@ -2703,7 +2718,6 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
             if (es != BTE_OK) return es;
         }
         BTE_CUDA(cudaEventRecord(ev[3], st));
-        BTE_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_margin.p, sizeof(double), cudaMemcpyDeviceToHost, st));
         if (aa_slots)
             BTE_CUDA(cudaMemcpyAsync(ctx->h_pinned + 1, ctx->d_aa_flag.p, sizeof(double), cudaMemcpyDeviceToHost, st));
         BTE_CUDA(cudaStreamSynchronize(st));

@@ -170,6 +170,14 @@ __global__ void k_diffuse_wall(const double* __restrict__ e_prev, const int* __r
 //   Tb[b][c] = sum_d e Omega_d / C_b + T_ref
 //   margin partial[b][block] = sum_d (e_curr - e_prev)^2 over the block's cells
 // (without MARGIN the sweep has already summed the margin partials).
+// The division by C_b costs an SM's FP64 pipe as much as four directions; it is
+// the same divisor for the block, so its reciprocal is formed once.
+// a / b for finite a and b with rb = 1 / b rounded, correctly rounded but for
+// over- and underflow (Markstein's theorem: one residual step); 3 operations.
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q = a * rb;
+    return fma(fma(-q, b, a), rb, q);
+}
 template <bool MARGIN>
 __global__ void __launch_bounds__(THREADS) k_reduce(const double* __restrict__ e_curr, const double* __restrict__ e_prev,
                                                     const double* __restrict__ omega, const double* __restrict__ Cb,
@@ -178,6 +186,7 @@ __global__ void __launch_bounds__(THREADS) k_reduce(const double* __restrict__ e
     __shared__ double sm[1][NWARP];
     const int c = blockIdx.x * THREADS + threadIdx.x;
     const int b = blockIdx.y;
+    const double cb = Cb[b], inv = 1.0 / cb;
     double m[1] = {0.0};
     if (c < n) {
         const double* ec = e_curr + (size_t)b * n_dir * Np + c;
@@ -192,7 +201,7 @@ __global__ void __launch_bounds__(THREADS) k_reduce(const double* __restrict__ e
                 m[0] = fma(df, df, m[0]);
             }
         }
-        Tb[(size_t)b * Np + c] = e0 / Cb[b] + T_ref;
+        Tb[(size_t)b * Np + c] = div_by(e0, cb, inv) + T_ref;
     }
     if (MARGIN) {
         block_sum<1>(m, sm);
@@ -204,20 +213,22 @@ __global__ void __launch_bounds__(THREADS) k_reduce(const double* __restrict__ e
 // ebar[b][c] = C_b / Omega_tot (T[c] - T_ref).  A block covers 32 cells with
 // 8 band slices (thread (x, y): cell x, bands y, y + 8, ...), so every load and
 // store is coalesced along the cells and the grid has n / 32 blocks; the 8
-// slice sums are added in slice order.
-constexpr int RC_CELLS = 32, RC_SLICES = 8;
+// slice sums are added in slice order.  C_b / Omega_tot is formed once per
+// block, RC_BANDS bands at a time, not by every thread.
+constexpr int RC_CELLS = 32, RC_SLICES = 8, RC_BANDS = 64;
 __global__ void __launch_bounds__(RC_CELLS * RC_SLICES)
     k_recover(const double* __restrict__ Tb, const double* __restrict__ Cb, const double* __restrict__ Lr,
               double Lr_sum, double T_ref, double solid_angle, int n, int n_band, size_t Np, double* T,
               double* ebar) {
     __shared__ double part[RC_SLICES][RC_CELLS];
-    __shared__ double tc[RC_CELLS];
+    __shared__ double tc[RC_CELLS], cs[RC_BANDS];
     const int x = threadIdx.x % RC_CELLS, y = threadIdx.x / RC_CELLS;
     const int c = blockIdx.x * RC_CELLS + x;
     double acc = 0.0;
     if (c < n)
         for (int b = y; b < n_band; b += RC_SLICES) acc += Lr[b] * Tb[(size_t)b * Np + c];
     part[y][x] = acc;
+    if ((int)threadIdx.x < min(n_band, RC_BANDS)) cs[threadIdx.x] = Cb[threadIdx.x] / solid_angle;
     __syncthreads();
     if (y == 0) {
         double t = 0.0;
@@ -226,9 +237,16 @@ __global__ void __launch_bounds__(RC_CELLS * RC_SLICES)
         if (c < n) T[c] = tc[x];
     }
     __syncthreads();
-    if (c < n) {
-        const double Tc = tc[x];
-        for (int b = y; b < n_band; b += RC_SLICES) ebar[(size_t)b * Np + c] = Cb[b] / solid_angle * (Tc - T_ref);
+    const double theta = tc[x] - T_ref;
+    for (int b0 = 0; b0 < n_band; b0 += RC_BANDS) {
+        const int nb = min(RC_BANDS, n_band - b0);
+        if (b0) {
+            __syncthreads();
+            if ((int)threadIdx.x < nb) cs[threadIdx.x] = Cb[b0 + threadIdx.x] / solid_angle;
+            __syncthreads();
+        }
+        if (c < n)
+            for (int b = y; b < nb; b += RC_SLICES) ebar[(size_t)(b0 + b) * Np + c] = cs[b] * theta;
     }
 }
 
@@ -241,6 +259,134 @@ __global__ void __launch_bounds__(THREADS) k_margin_final(const double* part, in
     for (int i = threadIdx.x; i < nparts; i += THREADS) v[0] += part[i];
     block_sum<1>(v, sm);
     if (threadIdx.x == 0) out[0] = v[0] / denom;
+}
+
+// k_reduce, k_recover and k_margin_final in one launch, for small states.
+// What bounds those there: the FP64 pipe (57 cycles of an SM per warp and
+// direction) on the few SMs that k_reduce's blocks of 256 cells reach, and three
+// launches.  A block here takes 32 cells, one per lane, with all bands and
+// directions, so T and ebar of its cells follow in it, and the last block to
+// finish adds the margin's partials.  Warp w sums the bands w, w + 8, ..., each
+// over the directions in order, as k_reduce.  Fewer than RC_SPLIT bands would
+// leave most warps idle and one with a chain of n_dir dependent sums: then the
+// warps take equal shares of the (band, direction) rows in order.
+struct ReduceArgs {
+    const double *e_curr, *e_prev, *omega, *Cb, *Lr;
+    double Lr_sum, T_ref, solid_angle;
+    int n, n_band, n_dir;
+    size_t Np;
+    double *Tb, *T, *ebar;
+    double* part;         // MARGIN: [blocks] margin partials
+    const double* mpart;  // else: the sweep's, nmpart of them
+    int nmpart;
+    unsigned* count;      // blocks that have finished; 0 before and after
+    double* margin;
+};
+constexpr int RC_LOADS = 8;  // directions whose loads are in flight together
+constexpr int RC_SPLIT = 4;  // bands from which a band is one warp's
+__host__ __device__ constexpr int reduce_groups(int n) { return (n + RC_CELLS - 1) / RC_CELLS; }
+// Where it is the faster one (us in all, three launches -> this one): up to two
+// blocks per SM, with fewer than RC_SPLIT bands (578 triangles x 1 band 24 -> 12,
+// 7,200 x 1 24 -> 13, 750 tetrahedra x 1 53 -> 16, 4,374 x 1 58 -> 18, 3,072 x 3 57 ->
+// 30) or up to kReduceRows rows a cell (1,058 triangles x 5 bands 24 -> 22, 10,082 x
+// 8 36 -> 32; beyond: 2,450 x 16 29 -> 37, 20,000 x 8 55 -> 61, 100,352 x 20 414 ->
+// 460, where k_reduce's rows of 2,048 bytes and blocks without a barrier win).
+constexpr int kReduceRows = 256, kReduceGroups = 320;
+inline bool reduce_by_cells(int n, int n_band, int n_dir) {
+    return reduce_groups(n) <= kReduceGroups && n_band <= RC_BANDS &&
+           (n_band < RC_SPLIT || (long long)n_band * n_dir <= kReduceRows);
+}
+
+template <bool MARGIN>
+__global__ void __launch_bounds__(RC_CELLS * RC_SLICES) k_reduce_cells(ReduceArgs a) {
+    static_assert(RC_CELLS * RC_SLICES == THREADS && RC_SPLIT + RC_SLICES <= RC_BANDS, "");
+    __shared__ double seg[RC_BANDS][RC_CELLS];  // band b's sum; in shares: warp w's of it in row b + w
+    __shared__ double slice[RC_SLICES][RC_CELLS];
+    __shared__ double inv[RC_BANDS], cs[RC_BANDS];  // 1 / C_b, C_b / Omega_tot
+    __shared__ double sm[1][NWARP];
+    __shared__ bool last;
+    const int lane = threadIdx.x % RC_CELLS, w = threadIdx.x / RC_CELLS, ND = a.n_dir, NB = a.n_band;
+    const int c = blockIdx.x * RC_CELLS + lane, rows = NB * ND;
+    const bool in = c < a.n, split = NB < RC_SPLIT;
+    double m[1] = {0.0}, acc = 0.0;
+    if ((int)threadIdx.x < NB) {
+        inv[threadIdx.x] = 1.0 / a.Cb[threadIdx.x];
+        cs[threadIdx.x] = a.Cb[threadIdx.x] / a.solid_angle;
+    }
+    for (int t = split ? rows * w / RC_SLICES : w * ND, t1 = split ? rows * (w + 1) / RC_SLICES : rows; t < t1;) {
+        const int b = t / ND, d = t - b * ND, k1 = min(ND - d, t1 - t);
+        const size_t at = (size_t)t * a.Np + c;
+        double e0 = 0.0;
+        if (in) {
+            for (int k0 = 0; k0 < k1; k0 += RC_LOADS) {
+                double v[RC_LOADS], p[RC_LOADS], o[RC_LOADS];
+#pragma unroll
+                for (int r = 0; r < RC_LOADS; ++r) {
+                    const int k = min(k0 + r, k1 - 1);
+                    v[r] = __ldcs(a.e_curr + at + (size_t)k * a.Np);
+                    if (MARGIN) p[r] = __ldcs(a.e_prev + at + (size_t)k * a.Np);
+                    o[r] = a.omega[d + k];
+                }
+#pragma unroll
+                for (int r = 0; r < RC_LOADS; ++r) {
+                    if (k0 + r >= k1) break;
+                    e0 += v[r] * o[r];
+                    if (MARGIN) {
+                        const double df = v[r] - p[r];
+                        m[0] = fma(df, df, m[0]);
+                    }
+                }
+            }
+        }
+        seg[split ? b + w : b][lane] = e0;
+        t += split ? k1 : RC_SLICES * ND;
+    }
+    __syncthreads();
+    for (int b = w; b < NB; b += RC_SLICES) {
+        double e0 = split ? 0.0 : seg[b][lane];
+        for (int u = 0; split && u < RC_SLICES; ++u) {
+            const int lo = rows * u / RC_SLICES, hi = rows * (u + 1) / RC_SLICES;
+            if (lo < (b + 1) * ND && hi > max(b * ND, lo)) e0 += seg[b + u][lane];
+        }
+        const double tb = div_by(e0, a.Cb[b], inv[b]) + a.T_ref;
+        if (in) a.Tb[(size_t)b * a.Np + c] = tb;
+        acc += a.Lr[b] * tb;
+    }
+    slice[w][lane] = acc;
+    __syncthreads();
+    if (w == 0) {
+        double t = 0.0;
+        for (int k = 0; k < RC_SLICES; ++k) t += slice[k][lane];
+        t /= a.Lr_sum;
+        if (in) a.T[c] = t;
+        slice[0][lane] = t - a.T_ref;
+    }
+    __syncthreads();
+    const double theta = slice[0][lane];
+    if (in)
+        for (int b = w; b < NB; b += RC_SLICES) a.ebar[(size_t)b * a.Np + c] = cs[b] * theta;
+    if (MARGIN) {
+        block_sum<1>(m, sm);
+        if (threadIdx.x == 0) {
+            a.part[blockIdx.x] = m[0];
+            __threadfence();
+            last = atomicAdd(a.count, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+    } else if (blockIdx.x != 0) {
+        return;
+    }
+    const double* part = MARGIN ? a.part : a.mpart;
+    const int nparts = MARGIN ? (int)gridDim.x : a.nmpart;
+    double v[1] = {0.0};
+    for (int i = threadIdx.x; i < nparts; i += THREADS) v[0] += __ldcg(part + i);
+    block_sum<1>(v, sm);
+    if (threadIdx.x == 0) {
+        *a.margin = v[0] / ((double)NB * a.n);
+        if (MARGIN) *a.count = 0;
+    }
 }
 
 // Heat flux, step 1 (src/StaticBTESolver.cpp:331-354): per (band, boundary face),
