@@ -2868,15 +2868,16 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
     if (o.max_iter == 0) result = BTE_OK;
     // heat flux (src/StaticBTESolver.cpp:323-370)
     if (ctx->nbf > 0) {
-        const int nt = ctx->nbf * NB;
-        BTE_LAUNCH(KK_HEAT, -1, (double)nt * ND * 16.0, 0,
-                   bte::k_heat_face<<<(nt + 127) / 128, 128, 0, st>>>(ctx->e_curr, ctx->d_bf_cell.as<int>(),
-                                                                    ctx->d_hw.as<double>(), ctx->nbf, NB, ND, Np,
-                                                                    ctx->d_hpart.as<double>()));
+        BTE_LAUNCH(KK_HEAT, -1, (double)ctx->nbf * NB * ND * 16.0, 0,
+                   bte::k_heat_face<<<dim3((ctx->nbf + bte::HF_FACES - 1) / bte::HF_FACES, NB),
+                                      bte::HF_FACES * bte::HF_PARTS, 0, st>>>(
+                       ctx->e_curr, ctx->d_bf_cell.as<int>(), ctx->d_hw.as<double>(), ctx->nbf, ND, Np,
+                       ctx->d_hpart.as<double>()));
     }
-    bte::k_heat_final<<<1, 256, 0, st>>>(ctx->d_hpart.as<double>(), ctx->d_bf_bc.as<int>(),
-                                        ctx->d_bf_area.as<double>(), ctx->d_vg.as<double>(), ctx->nbf, NB,
-                                        ctx->n_bc, ctx->dim, ctx->d_qband.as<double>(), ctx->d_q.as<double>());
+    if (ctx->n_bc > 0)
+        bte::k_heat_final<<<ctx->n_bc, bte::THREADS, 0, st>>>(
+            ctx->d_hpart.as<double>(), ctx->d_bf_bc.as<int>(), ctx->d_bf_area.as<double>(), ctx->d_vg.as<double>(),
+            ctx->nbf, NB, ctx->dim, ctx->d_qband.as<double>(), ctx->d_q.as<double>());
     BTE_LAUNCHED();
     int dsa_stat[4] = {0, 0, 0, 0};
     if (dsa_on && rep.dsa_solves > 0)
