@@ -2323,6 +2323,14 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
     return BTE_OK;
 }
 
+// ebar for the kernels that follow a sweep or Krylov batch, or null when nothing
+// reads it: the stream sweep of an acyclic plan (no residual kernel) forms it
+// from T.  To be asked after the solve's first sweep, which chooses the kernel.
+static double* read_ebar(const bte_ctx* ctx, int form) {
+    const bool unread = form == BTE_FORM_SWEEP && ctx->sweep_shape.stream && ctx->plan_lagged_dirs == 0;
+    return unread ? nullptr : ctx->d_ebar.as<double>();
+}
+
 // Anderson state: T and the intensities at the cells with boundary faces.
 static bte::mlp::AaState aa_state(const bte_ctx* ctx) {
     return bte::mlp::AaState{ctx->d_bcell.as<int>(), ctx->n, ctx->nbcell, ctx->n_band, ctx->n_dir, ctx->Np,
@@ -2334,8 +2342,8 @@ static size_t aa_len(const bte_ctx* ctx) { return (size_t)ctx->n + (size_t)ctx->
 // iteration, form the Gram matrix of the stored f, solve for alpha and set
 // T = sum alpha_i g_i (and ebar).  The history restarts when the margin grew
 // tenfold or the weights blow up.
-static bte_status anderson_step(bte_ctx* ctx, int slots, int& count, int& next, std::vector<int>& order, double m,
-                                bte_report& rep) {
+static bte_status anderson_step(bte_ctx* ctx, int form, int slots, int& count, int& next, std::vector<int>& order,
+                                double m, bte_report& rep) {
     namespace M = bte::mlp;
     cudaStream_t st = ctx->stream;
     const int n = ctx->n;
@@ -2375,10 +2383,10 @@ static bte_status anderson_step(bte_ctx* ctx, int slots, int& count, int& next, 
                M::k_aa_mix<<<gl, 256, 0, st>>>(as, ctx->d_aa_g.as<double>(), L, mx, ctx->d_aa_alpha.as<double>(),
                                                 ctx->T_ref, ctx->d_T.as<double>(), ctx->d_ebar.as<double>(),
                                                 ctx->e_curr));
-    BTE_LAUNCH(KK_REDUCE, -1, (double)(ctx->n_band + 1) * n * 8.0, 0,
-               M::k_ebar_from_T<<<dim3((n + 255) / 256, ctx->n_band), 256, 0, st>>>(
-                   ctx->d_T.as<double>(), ctx->d_Cb.as<double>(), ctx->solid_angle, ctx->T_ref, n, ctx->Np,
-                   ctx->d_ebar.as<double>()));
+    if (double* ebar = read_ebar(ctx, form))
+        BTE_LAUNCH(KK_REDUCE, -1, (double)(ctx->n_band + 1) * n * 8.0, 0,
+                   M::k_ebar_from_T<<<dim3((n + 255) / 256, ctx->n_band), 256, 0, st>>>(
+                       ctx->d_T.as<double>(), ctx->d_Cb.as<double>(), ctx->solid_angle, ctx->T_ref, n, ctx->Np, ebar));
     ++rep.accel_steps;
     return BTE_OK;
 }
@@ -2647,7 +2655,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
             if (ctx->dim != 1 && bte::reduce_by_cells(ctx->n, NB, ND)) {  // (1D Krylov solves follow the last bit, see batch_len)
                 const bte::ReduceArgs ra{ctx->e_curr, ctx->e_prev, ctx->d_omega.as<double>(), ctx->d_Cb.as<double>(),
                                          ctx->d_Lr.as<double>(), Lr_sum, ctx->T_ref, ctx->solid_angle, ctx->n, NB, ND,
-                                         Np, ctx->d_Tb.as<double>(), ctx->d_T.as<double>(), ctx->d_ebar.as<double>(),
+                                         Np, ctx->d_Tb.as<double>(), ctx->d_T.as<double>(), read_ebar(ctx, o.form),
                                          ctx->d_mpart.as<double>(), ctx->d_spart.as<double>(), ND * NB,
                                          ctx->d_count.as<unsigned>(), ctx->h_pinned};
                 const int groups = bte::reduce_groups(ctx->n);
@@ -2671,7 +2679,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
                        bte::k_recover<<<(ctx->n + bte::RC_CELLS - 1) / bte::RC_CELLS, bte::RC_CELLS * bte::RC_SLICES,
                                         0, st>>>(
                            ctx->d_Tb.as<double>(), ctx->d_Cb.as<double>(), ctx->d_Lr.as<double>(), Lr_sum, ctx->T_ref,
-                           ctx->solid_angle, ctx->n, NB, Np, ctx->d_T.as<double>(), ctx->d_ebar.as<double>()));
+                           ctx->solid_angle, ctx->n, NB, Np, ctx->d_T.as<double>(), read_ebar(ctx, o.form)));
             // margin = sum of the partials / (n_band n_cell), fixed order
             bte::k_margin_final<<<1, bte::THREADS, 0, st>>>(fused ? ctx->d_spart.as<double>() : ctx->d_mpart.as<double>(),
                                                             fused ? ND * NB : nred * NB, (double)NB * ctx->n,
@@ -2800,7 +2808,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
             BTE_LAUNCH(KK_DSA, -1, (2.0 + NB) * n * 8.0, 0,
                        bte::dsa::k_dsa_apply<<<(n + 255) / 256, 256, 0, st>>>(
                            ctx->d_dsa_x.as<double>(), ctx->d_dsa_pos.as<int>(), ctx->d_Cb.as<double>(),
-                           ctx->solid_angle, ctx->T_ref, n, NB, Np, ctx->d_T.as<double>(), ctx->d_ebar.as<double>(),
+                           ctx->solid_angle, ctx->T_ref, n, NB, Np, ctx->d_T.as<double>(), read_ebar(ctx, o.form),
                            ctx->d_dsa_xc.as<double>()));
             if (ctx->nbcell > 0) {
                 const int nt = ctx->nbcell * ND;
@@ -2814,7 +2822,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
             ++rep.dsa_solves;
         }
         if (aa_slots && it > 0) {
-            bte_status s = anderson_step(ctx, aa_slots, aa_count, aa_next, aa_order, m, rep);
+            bte_status s = anderson_step(ctx, o.form, aa_slots, aa_count, aa_next, aa_order, m, rep);
             if (s != BTE_OK) return s;
         }
         if ((o.accel == 1 || o.accel == 2) && accel_on && accel_last >= 0 && it == accel_last + o.accel_every - 1 &&
@@ -2850,7 +2858,7 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
                        bte::mlp::k_accel_apply<<<(n + 255) / 256, 256, 0, st>>>(
                            ctx->d_ring.as<double>(), s0, s1, s2, Np, n, ctx->d_scale.as<double>(),
                            ctx->d_y.as<float>(), o.accel == 1, ctx->d_Cb.as<double>(), NB, ctx->solid_angle,
-                           ctx->T_ref, ctx->d_T.as<double>(), ctx->d_ebar.as<double>()));
+                           ctx->T_ref, ctx->d_T.as<double>(), read_ebar(ctx, o.form)));
             accel_last = it;
             accel_margin = m;
             ++rep.accel_steps;

@@ -698,6 +698,7 @@ __global__ void k_dsa_rhs(const double* __restrict__ T, const double* __restrict
 
 // T += x, and the equilibrium energy density follows: ebar[b][c] = C_b / Omega_tot (T - T_ref).
 // x is in the solve's numbering (pos[c] = position of cell c); xc[c] receives it by cell.
+// ebar null: nothing reads it (k_recover).
 __global__ void k_dsa_apply(const double* __restrict__ x, const int* __restrict__ pos, const double* __restrict__ Cb,
                             double solid_angle, double T_ref, int n, int n_band, size_t Np, double* __restrict__ T,
                             double* __restrict__ ebar, double* __restrict__ xc) {
@@ -707,7 +708,7 @@ __global__ void k_dsa_apply(const double* __restrict__ x, const int* __restrict_
     xc[c] = dx;
     const double t = T[c] + dx;
     T[c] = t;
-    for (int b = 0; b < n_band; ++b) ebar[(size_t)b * Np + c] = Cb[b] / solid_angle * (t - T_ref);
+    for (int b = 0; ebar && b < n_band; ++b) ebar[(size_t)b * Np + c] = Cb[b] / solid_angle * (t - T_ref);
 }
 
 // The intensities of the cells with boundary faces, which the next outer

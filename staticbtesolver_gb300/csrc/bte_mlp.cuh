@@ -567,7 +567,7 @@ __global__ void k_accel_apply(const double* __restrict__ ring, int s0, int s1, i
     if (learned) u = fmin(64.0, fmax(-64.0, u + fmin(8.0, fmax(-8.0, (double)y[c]))));
     const double Tn = t0 + s * u;
     T[c] = Tn;
-    for (int b = 0; b < n_band; ++b) ebar[(size_t)b * Np + c] = Cb[b] / solid_angle * (Tn - T_ref);
+    for (int b = 0; ebar && b < n_band; ++b) ebar[(size_t)b * Np + c] = Cb[b] / solid_angle * (Tn - T_ref);
 }
 
 // ---------------------------------------------------------------------------
