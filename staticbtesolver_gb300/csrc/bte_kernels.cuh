@@ -51,6 +51,13 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double (*smem)[NWARP])
         }
 }
 
+// a / b for finite a and b with rb = 1 / b rounded, correctly rounded but for
+// over- and underflow (Markstein's theorem: one residual step); 3 operations.
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q = a * rb;
+    return fma(fma(-q, b, a), rb, q);
+}
+
 // Serial sum of the per-chunk partials (for kernels with one thread per system).
 __device__ __forceinline__ double sum_parts_serial(const double* p, int n) {
     double s = 0;

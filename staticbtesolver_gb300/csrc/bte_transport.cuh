@@ -172,12 +172,6 @@ __global__ void k_diffuse_wall(const double* __restrict__ e_prev, const int* __r
 // (without MARGIN the sweep has already summed the margin partials).
 // The division by C_b costs an SM's FP64 pipe as much as four directions; it is
 // the same divisor for the block, so its reciprocal is formed once.
-// a / b for finite a and b with rb = 1 / b rounded, correctly rounded but for
-// over- and underflow (Markstein's theorem: one residual step); 3 operations.
-__device__ __forceinline__ double div_by(double a, double b, double rb) {
-    const double q = a * rb;
-    return fma(fma(-q, b, a), rb, q);
-}
 template <bool MARGIN>
 __global__ void __launch_bounds__(THREADS) k_reduce(const double* __restrict__ e_curr, const double* __restrict__ e_prev,
                                                     const double* __restrict__ omega, const double* __restrict__ Cb,
