@@ -1496,12 +1496,21 @@ static bte_status batch_outcome(bte_ctx* ctx, int S, bte_report& rep) {
 // kernels; so does BTE_KRYLOV=phase, and =persistent its own kernel.  1D keeps
 // the phase kernels and their rounding: there r_hat . r falls to rounding level
 // within a few steps, some systems of every run end at the iteration limit, and
-// which ones do depends on the last bit of every sum.
+// which ones do depends on the last bit of every sum.  So it is for large PLAIN
+// systems without scattering: of 512 solves per run, on 8,192 to 20,000 triangles
+// with mean free paths above the side, one in ten runs (8,192) to one in three
+// (20,000) has a system at the limit, from either kernel and seldom the same one,
+// which moves the field by 1e-8 to 1e-4; up to 5,000 none did in 64 runs.  PLAIN
+// takes clusters up to kClusterPlain cells (20,000 x 256 systems would go from 192
+// to 83 ms); MIXED, whose refinement ends every system, up to their full size.
+constexpr int kClusterPlain = 4096;
 template <typename Op, typename T>
 static bte_status batch_len(bte_ctx* ctx, int S, int prec, int* len) {
     *len = 0;
     const char* v = std::getenv("BTE_KRYLOV");
-    if (ctx->profile || (v && v[0] == 'p') || ctx->dim == 1 || ctx->n > bte::KC_CELLS * bte::KC_CTAS) return BTE_OK;
+    if (ctx->profile || (v && v[0] == 'p') || ctx->dim == 1 ||
+        ctx->n > (prec == 0 ? kClusterPlain : bte::KC_CELLS * bte::KC_CTAS))
+        return BTE_OK;
     if (ctx->kc_slots == 0) {  // face slots: the largest inflow count
         BTE_CUDA(ctx->m_active.alloc(sizeof(int)));
         BTE_CUDA(cudaMemsetAsync(ctx->m_active.p, 0, sizeof(int), ctx->stream));

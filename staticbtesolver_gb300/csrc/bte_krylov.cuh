@@ -27,8 +27,8 @@
 //  * one warp per CTA forms the iteration's scalars.
 // Solves measured, phase kernels -> clusters: 578 triangles x 32 directions to
 // margin 1e-5, 135 -> 17.4 ms; 750 tetrahedra x 128 directions, 228 -> 43 ms;
-// 20,000 triangles x 256 systems, two outer iterations, 199 -> 84 ms; 10,082
-// triangles x 256 systems in mixed precision, three, 157 -> 25 ms.  One CSR
+// 10,082 triangles x 256 systems in mixed precision, three outer iterations, 157
+// -> 25 ms (FP64 beyond 4,096 cells keeps the phase kernels, batch_len).  One CSR
 // system from host arrays, to 1e-12: 968 unknowns 2.8 -> 0.56 ms, 9,800 unknowns
 // 10.0 -> 1.9 ms (9 us a step: 3.7 of the FP64 pipe, the rest barriers and remote
 // loads), 32,768 unknowns 20.5 -> 5.6 ms.

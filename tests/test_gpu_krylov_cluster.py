@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 # one cell more or less than a row of 256 threads, a full CTA and the largest
 # cluster; systems few enough to spread over several CTAs, and many
-CELLS = [1, 2, 33, 255, 256, 257, 2047, 2048, 2049, 4097, 20000, 32767, 32768, 32769]
+CELLS = [1, 2, 33, 255, 256, 257, 2047, 2048, 2049, 4096, 4097, 20000, 32767, 32768, 32769]
 MESHES = [("square16_b8", 0), ("square10_b40", 0), ("2DM2DG", 0), ("3DM2DG", 0), ("cube4_b2", 0), ("cube7_b1", 4),
           ("cube14_b1", 2)]
 
@@ -51,7 +51,8 @@ def test_cluster_equals_phase_kernels(sbte, get_case, tmp_path, name, max_iter, 
         p = synth.make_problem(name, str(tmp_path))
         args, limit = (p.geo, p.bc_file, p.band_file, p.DM, p.num_theta, p.num_phi, p.T_ref, p.L_x, p.L_y, p.L_z), 1000
     r0, r1 = _both(sbte, sbte.Problem(*args), max_iter=max_iter or limit, form=getattr(sbte, "FORM_" + form))
-    assert r1["kernel_launches"] < r0["kernel_launches"]  # one launch instead of five per iteration
+    if form == "MIXED" or name != "cube14_b1":  # (FP64 beyond 4,096 cells: the phase kernels)
+        assert r1["kernel_launches"] < r0["kernel_launches"]  # one launch instead of five per iteration
 
 
 @pytest.fixture(scope="module")
@@ -73,7 +74,7 @@ def test_cluster_cell_counts(sbte, wide_mesh, cells, form):
         a[k] = a[k][:cells]
     a["nbr"] = np.where(a["nbr"] >= cells, -1, a["nbr"])
     r0, r1 = _both(sbte, a, max_iter=2, tol_=0.0, form=getattr(sbte, "FORM_" + form))
-    if cells <= 32768:
+    if cells <= (4096 if form == "PLAIN" else 32768):
         assert r1["kernel_launches"] < r0["kernel_launches"]
 
 
