@@ -85,6 +85,21 @@ private:
     size_t size = 0;
 };
 
+// Lets kernel k be launched with `bytes` of dynamic shared memory, or fails when
+// the device has less.  The limit belongs to the kernel on the device, not to a
+// context or a thread, and a launch above it is refused: so it only ever takes
+// one value, all that the device allows beside the kernel's static memory.
+inline cudaError_t allow_smem(const void* k, int device, size_t bytes) {
+    int most = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) return e;
+    most -= (int)a.sharedSizeBytes;
+    return bytes > (size_t)most ? cudaErrorInvalidValue
+                                : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 constexpr int kGroup = 8;  // BiCGSTAB iterations launched between host checks
 
 enum KernelKind { KK_P, KK_SPMV1, KK_S, KK_SPMV2, KK_X, KK_INIT, KK_RHS, KK_REDUCE, KK_DIFFUSE, KK_HEAT, KK_SWEEP,
@@ -910,8 +925,7 @@ static bte_status dsa_upload(bte_ctx* ctx, DsaHostPlan& hp, cudaStream_t st) {
         const int kgb = bte::dsa::kGjBlock;
         const size_t smem_blk = sizeof(double) * (size_t)kgb * (m + kgb + 1);
         if (coop_ok && smem_blk + 1024 <= (size_t)smem_opt) {
-            BTE_CUDA(cudaFuncSetAttribute(bte::dsa::k_gj_block_all, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem_blk));
+            BTE_CUDA(allow_smem((const void*)bte::dsa::k_gj_block_all, ctx->device, smem_blk));
             BTE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_blk, bte::dsa::k_gj_block_all, 1024, smem_blk));
         }
         if (occ_blk >= 1) {
@@ -967,7 +981,7 @@ static bte_status dsa_upload(bte_ctx* ctx, DsaHostPlan& hp, cudaStream_t st) {
     ctx->dsa_topo = with_topo + 16384 <= (size_t)smem_max;
     if (ctx->dsa_topo) ctx->dsa_smem = with_topo;
     auto pcg = ctx->dsa_topo ? bte::dsa::k_dsa_pcg<true> : bte::dsa::k_dsa_pcg<false>;
-    BTE_CUDA(cudaFuncSetAttribute(pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->dsa_smem));
+    BTE_CUDA(allow_smem((const void*)pcg, ctx->device, ctx->dsa_smem));
     BTE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pcg, kDsaThreads, ctx->dsa_smem));
     if (occ < 1 || nblk > occ * sms) return fail(ctx, BTE_ERR_CUDA, "dsa: the low-order kernel cannot be resident");
     BTE_CUDA(upload(ctx->d_lo_nb, nbv, st));
@@ -1179,8 +1193,7 @@ static bte_status build_sweep_plan(bte_ctx* ctx) {
         const int wcap = smem_state < room ? (int)std::min<size_t>({(size_t)8192, (size_t)n, (room - smem_state) / 4}) : 0;
         if (!level_order_global() && wcap >= std::min(n, 2048)) {
             const size_t smem = smem_state + sizeof(int) * (size_t)wcap;
-            BTE_CUDA(cudaFuncSetAttribute(bte::k_level_order_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+            BTE_CUDA(allow_smem((const void*)bte::k_level_order_smem, ctx->device, smem));
             bte::k_level_order_smem<<<ND, 1024, smem, st>>>(ctx->lo_mask.as<uint8_t>(), ctx->lo_down.as<int>(), n, F,
                                                             wcap, ctx->lo_perm.as<int>(), ctx->lo_lvl.as<int>(),
                                                             d_small, d_small + ND, d_small + 2 * ND);
@@ -1191,7 +1204,7 @@ static bte_status build_sweep_plan(bte_ctx* ctx) {
                 cap *= 2;
             const size_t smem = (size_t)2 * cap * sizeof(int);
             BTE_CUDA(ctx->lo_indeg.alloc(sizeof(int) * (size_t)ND * n));
-            BTE_CUDA(cudaFuncSetAttribute(bte::k_level_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            BTE_CUDA(allow_smem((const void*)bte::k_level_order, ctx->device, smem));
             bte::k_level_order<<<ND, 1024, smem, st>>>(ctx->lo_mask.as<uint8_t>(), ctx->lo_down.as<int>(), n, F, cap,
                                                        ctx->lo_indeg.as<int>(), ctx->lo_perm.as<int>(),
                                                        ctx->lo_lvl.as<int>(), d_small, d_small + ND, d_small + 2 * ND);
@@ -1457,7 +1470,7 @@ static int cluster_len(int device, int S, int n, int slots, bool best = true, in
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = cluster_config<T>(S, (n + len - 1) / len, len, slots, best, nullptr, &attr);
     int clusters = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+    if (allow_smem(k, device, cfg.dynamicSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
         cudaGetLastError();
