@@ -1,6 +1,6 @@
 """Contexts of different sizes alive at once, and calls of different sizes from several host threads:
-what a kernel may be launched with is no one problem's, and different contexts are independent: each solve gives what it gives alone, to the
-bit."""
+what a kernel may be launched with is no one problem's, and contexts are independent, so each solve
+gives what it gives alone, to the bit."""
 import threading
 
 import numpy as np
