@@ -115,21 +115,23 @@ typedef struct bte_report {
     double ms_reduce;          /* temperature / margin reductions and the accelerator */
     long long kernel_launches; /* kernels this library launched during the solve */
     int sweep_group;           /* sweep form: bands per block and threads per block, chosen by a model */
-    int sweep_threads;         /* of the launch (stream kernel) or by timing candidates on a plan's first sweep */
+    int sweep_threads;         /* of the launch or by timing candidates on a plan's first sweep */
     int accel_steps;           /* outer-iteration extrapolations (accel 1, 2) or mixes (3) applied */
     int accel_reverts;         /* extrapolations undone (state restored) */
     int sweep_ring;            /* sweep form: solved positions kept in shared memory per band */
     int sweep_margin;          /* sweep form, acyclic plan: 1 the sweep sums the margin, 0 the reduction
-                                  does (always with the stream kernel; else timed with the launch shape) */
+                                  does (always with the stream kernel; else modelled or timed with the
+                                  launch shape) */
     int dsa_solves;            /* low-order corrections applied (dsa) */
     long long dsa_iterations;  /* conjugate-gradient iterations summed over them */
     double ms_dsa;             /* device time of the corrections (included in ms_reduce and ms_total) */
     int sweep_kernel;          /* sweep form: the kernel that ran -- 3 stream (k_sweep_stream: everything but
-                                  the solution brought to shared memory ahead), taken whenever the plan
-                                  suits it; else the autotuner's choice: 0 level-synchronous (k_sweep), 1
-                                  staged (levels copied to shared memory ahead by bulk copies), 2
-                                  level-synchronous over levels split into slices of one position per
-                                  thread */
+                                  the solution brought to shared memory ahead) or 0 level-synchronous
+                                  (k_sweep, which sums the margin too: the faster one for many directions
+                                  or bands on few cells), by models of both; where the plan does not suit
+                                  the stream kernel the autotuner's choice among 0, 1 staged (levels
+                                  copied to shared memory ahead by bulk copies) and 2 level-synchronous
+                                  over levels split into slices of one position per thread */
     double ms_host_setup;      /* host wall time of this call's set-up after new inputs (uploads, geometry) */
     double ms_host_plan;       /* ... of building the sweep plan (level order, layout) after new geometry */
     double ms_host_order;      /*     of which the level order (host threads over directions) */
@@ -263,8 +265,8 @@ bte_status bte_mlp_train(const float* X, const float* Y, int M, int steps, int b
 bte_status bte_get_kernel_stats(bte_ctx* ctx, bte_kernel_stat* stats, int cap, int* n);
 
 /* The sweep autotuner's table from the first sweep of the current plan (empty
- * when the stream kernel ran, whose shape is not timed, or the choice came from
- * the per-process cache): candidate k ran with
+ * when a model chose kernel and shape, which then are not timed, or the choice
+ * came from the per-process cache): candidate k ran with
  * group[k] bands and threads[k] threads per block and ring[k] positions per
  * band, with kernel[k] (0 level-synchronous, 1 staged, 2 split levels, as
  * bte_report.sweep_kernel), in ms[k] milliseconds.  Entries are written up

@@ -1992,86 +1992,205 @@ static bte_status stream_records(bte_ctx* ctx, const SweepShape& sh) {
     return BTE_OK;
 }
 
-// The stream kernel's shape for batches of nbb bands into ctx->sweep_shape;
-// *found = false: the plan does not suit it (levels so narrow that padding them
-// to rows would take more than the state itself and kStreamFree bytes, or so
-// wide that no ring holds a few of them).
+// f(positions of a level), summed over a direction's levels: the directions' mean
+// and the largest.
+struct PlanSum {
+    double mean = 0, most = 0;
+};
+template <typename F>
+static PlanSum plan_sum(const bte_ctx* ctx, F&& f) {
+    PlanSum s;
+    for (int d = 0; d < ctx->n_dir; ++d) {
+        const int l1 = ctx->plan_lvl_off[d + 1] - 1;
+        long long v = 0;
+        for (int l = ctx->plan_lvl_off[d]; l < l1; ++l) v += f(ctx->plan_lvl[l + 1] - ctx->plan_lvl[l]);
+        s.mean += (double)v / ctx->n_dir;
+        s.most = std::max(s.most, (double)v);
+    }
+    return s;
+}
+// A launch of `blocks` blocks, `fit` of them on an SM: its waves, of average
+// directions up to the last one's.  block(longest, share): cycles of a block of an
+// average or the longest direction, one of `share` on its SM.
+template <typename F>
+static double wave_cost(int blocks, int fit, int sms, F&& block) {
+    const int full = (blocks - 1) / (sms * fit);
+    return full * block(false, fit) + block(true, (blocks - full * sms * fit + sms - 1) / sms);
+}
+
+// The stream kernel's shape for batches of nbb bands with `annex` places per chunk in
+// *out and its cycles in *cost, or *cost = kNoShape: the plan does not suit it (levels
+// so narrow that padding them to rows would take more than the state itself and
+// kStreamFree bytes, or so wide that no ring holds a few of them).
 //
-// A model of the launch instead of timing candidates: its constants (cycles)
-// were fitted to 250 shapes on each of 18 plans (2D 128 to 100,352 triangles, 3D
-// 3,072 to 131,712 tetrahedra, 1 to 40 bands); the shape it picks takes 1.5 %
-// longer than the fastest one on average and 8 % at most, and a plan of a new
-// mesh costs no trial sweeps (before: ~20, 100 ms on 100,352 triangles).  Per
-// stage, the slowest of
-//  * a consumer warp's rows one after the other, with a barrier;
-//  * the FP64 pipe over the systems that share an SM;
-//  * the chunks' way through copy and helpers, NCH of them in flight;
-// times the waves of blocks.
+// A model of the launch instead of timing candidates.  A block takes the slowest of
+//  * a consumer warp's turns (a level of few rows takes a turn however many warps
+//    there are) and the levels' barriers, longer the more consumer warps share the SM;
+//  * the FP64 pipe over the systems that share an SM, with the idle warps' part;
+//  * the chunks' way through copy and helpers, who form every band's right-hand
+//    sides, NCH chunks in flight;
+//  * on tetrahedra, the bytes of records and coefficients.
+// The constants (cycles) were fitted to ~90 shapes on each of 189 plans (162 to
+// 39,200 triangles x 1 to 40 bands, 162 to 55,566 tetrahedra x 1 to 20 bands): the
+// shape picked takes 1.1 % (2D) and 1.4 % (3D) longer than the fastest on average, 8 %
+// and 15 % at most; on 18 other plans, up to 100,352 triangles and 131,712 tetrahedra,
+// 1 % and 8 %.  (With the mean rows per level in place of the turns and no helpers' time
+// per band it picked shapes up to 80 % longer: 16,464 tetrahedra x 16 bands 1,126 us,
+// now 666; 2,450 triangles x 24 bands 113 us, now 63.)  A plan of a new mesh costs no
+// trial sweeps (~20, 100 ms on 100,352 triangles).
 constexpr size_t kStreamFree = (size_t)256 << 20;
-static bte_status stream_choose(bte_ctx* ctx, int nbb, bool* found) {
-    *found = false;
+constexpr double kNoShape = 1e300;
+static bte_status stream_choose(bte_ctx* ctx, int nbb, int annex, SweepShape* out, double* cost) {
+    *cost = kNoShape;
     const int fm = sweep_slots(ctx), cap = ctx->stream_width;
     const size_t npad = (size_t)ctx->stream_nq * bte::SCH;
     if (cap <= 0 || (npad > 2 * ctx->Np && 16 * npad * ctx->n_band * ctx->n_dir > kStreamFree)) return BTE_OK;
-    static const double kRow[3] = {520, 850, 900}, kFp64[3] = {136, 171, 200};
-    constexpr double kBarrier = 100, kPipe = 11600;
+    // cycles per row of a warp's turn, per barrier, of the FP64 pipe per row, of a
+    // chunk's way and more of it per band, per byte, by face slots (four: not measured)
+    static const struct { double row, bar, fp64, crowd, more, way, band, byte; } kCost[3] = {
+        {545, 170, 104, 0.165, 0.13, 5700, 1700, 0}, {635, 220, 120, 0.22, 0.06, 7000, 2090, 0.095},
+        {670, 220, 140, 0.22, 0.06, 7000, 2090, 0.095}};
+    const size_t rec = fm == 2 ? bte::StreamRec<2>::bytes : fm == 3 ? bte::StreamRec<3>::bytes : bte::StreamRec<4>::bytes;
+    const auto& kc = kCost[fm - 2];
     int smem_max = 0, sms = 0, smem_sm = 0, regs_sm = 0, threads_sm = 0;
     BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     BTE_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
     BTE_CUDA(cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, ctx->device));
     BTE_CUDA(cudaDeviceGetAttribute(&threads_sm, cudaDevAttrMaxThreadsPerMultiProcessor, ctx->device));
     BTE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    long long rows = 0;
-    for (int d = 0; d < ctx->n_dir; ++d) rows += ctx->plan_lrow[ctx->plan_lvl_off[d + 1] - 1];
-    const double per = (double)rows / std::max(1ll, ctx->plan_levels);  // rows per level
-    for (int annex = cap / 16 + 8, tries = 0; tries < 4; ++tries) {
-        SweepShape best;
-        double best_cost = 1e300;
-        for (int nch = 4; nch <= 8; nch *= 2)
-            for (int G = 1; G <= std::min(nbb, 10); ++G)
-                for (int WC = 1; WC <= 6; ++WC) {
-                    SweepShape sh;
-                    sh.stream = true;
-                    sh.G = G;
-                    sh.WC = WC;
-                    sh.NCH = sh.H = nch;
-                    sh.cap = cap;
-                    sh.A = annex;
-                    // a ring of four or five of the widest levels: older values go
-                    // through the annexes (132,000 tetrahedra, levels up to 1,568:
-                    // 8,192 positions 6.3 ms, 4,096 7.1 ms)
-                    sh.W = 1024;
-                    while (sh.W < std::max(cap + (nch + 1) * bte::SCH, 9 * cap / 2)) sh.W <<= 1;
-                    sh.threads = 32 * (G * WC + nch + 1);
-                    sh.smem = stream_smem(fm, sh);
-                    if (sh.smem > (size_t)smem_max || sh.threads > bte::STHREADS ||
-                        !bte::stream_shape_ok(sh.stream_shape()))
-                        continue;
-                    const int fit = std::min({smem_sm / (int)(sh.smem + 1024), regs_sm / (80 * sh.threads),
-                                              threads_sm / sh.threads});
-                    if (fit < 1) continue;
-                    const int blocks = (nbb + G - 1) / G * ctx->n_dir;
-                    const int waves = (blocks + sms * fit - 1) / (sms * fit);
-                    const int share = std::min(fit, (blocks + sms - 1) / sms);  // blocks on the fullest SM
-                    const double cost = waves * std::max({(per / WC + 0.25) * kRow[fm - 2] + kBarrier,
-                                                          per * G * share * kFp64[fm - 2], per / 4 * kPipe / (nch - 1)});
-                    if (cost < best_cost) {
-                        best_cost = cost;
-                        best = sh;
-                    }
+    constexpr int kWarps = 6;
+    const PlanSum levels = plan_sum(ctx, [](int) { return 1; });
+    const PlanSum rows = plan_sum(ctx, [](int w) { return (w + 31) / 32; });
+    PlanSum turns[kWarps + 1];
+    for (int wc = 1; wc <= kWarps; ++wc)
+        turns[wc] = plan_sum(ctx, [wc](int w) { return ((w + 31) / 32 + wc - 1) / wc; });
+    for (int nch = 4; nch <= 8; nch *= 2)
+        for (int G = 1; G <= std::min(nbb, 10); ++G)
+            for (int WC = 1; WC <= kWarps; ++WC) {
+                SweepShape sh;
+                sh.stream = true;
+                sh.G = G;
+                sh.WC = WC;
+                sh.NCH = sh.H = nch;
+                sh.cap = cap;
+                sh.A = annex;
+                // a ring of four or five of the widest levels: older values go
+                // through the annexes (132,000 tetrahedra, levels up to 1,568:
+                // 8,192 positions 6.3 ms, 4,096 7.1 ms)
+                sh.W = 1024;
+                while (sh.W < std::max(cap + (nch + 1) * bte::SCH, 9 * cap / 2)) sh.W <<= 1;
+                sh.threads = 32 * (G * WC + nch + 1);
+                sh.smem = stream_smem(fm, sh);
+                if (sh.smem > (size_t)smem_max || sh.threads > bte::STHREADS ||
+                    !bte::stream_shape_ok(sh.stream_shape()))
+                    continue;
+                const int fit = std::min({smem_sm / (int)(sh.smem + 1024), regs_sm / (80 * sh.threads),
+                                          threads_sm / sh.threads});
+                if (fit < 1) continue;
+                const double c = wave_cost((nbb + G - 1) / G * ctx->n_dir, fit, sms, [&](bool longest, int share) {
+                    const auto of = [&](const PlanSum& v) { return longest ? v.most : v.mean; };
+                    return std::max({(of(turns[WC]) * kc.row + of(levels) * kc.bar) *
+                                         (1 + kc.crowd * (share * G * WC - 1) / 16),
+                                     of(rows) * share * G * kc.fp64 * (1 + kc.more * (WC - 1)),
+                                     of(rows) / 4 * (kc.way + kc.band * G) / nch,
+                                     of(rows) * share * 32 * (double)(rec + 16 * G) * kc.byte});
+                });
+                if (c < *cost) {
+                    *cost = c;
+                    *out = sh;
                 }
-        if (!(best_cost < 1e300)) return BTE_OK;
-        bte_status s = stream_plan(ctx);
-        if (s == BTE_OK) s = stream_annex(ctx, best);
-        if (s != BTE_OK) return s;
-        if (best.smem <= (size_t)smem_max) {
-            ctx->sweep_shape = best;
+            }
+    return BTE_OK;
+}
+
+// k_sweep's shape for batches of nbb bands on an acyclic plan in *out; returns its
+// cycles, with `margin`, what the closing reduction takes longer when the sweep does
+// not sum the margin.  A block takes the slowest of its rounds of 128 threads through
+// the levels and the FP64 pipe over the warps' steps of the blocks on its SM.  A ring
+// of less than six of the widest levels is not taken (kNoShape if none is longer):
+// older upstream values cost two dependent loads each (29,478 tetrahedra x 12 bands,
+// levels up to 608: one band a block 1,199 us, four 2,379).  Fitted to 212 plans, 32 to 512 directions: where it
+// is the faster kernel the estimate is within 15 %.
+static double level_choose(bte_ctx* ctx, int nbb, int sms, double margin, SweepShape* out) {
+    static const struct { double round, crowd, fp64, sum; } kCost[2] = {{1360, 0.06, 167, 41}, {1520, 0.037, 173, 37}};
+    const auto& kc = kCost[sweep_slots(ctx) > 2];
+    constexpr int kThreads = 128, kFit = 5;
+    double best = kNoShape;
+    for (int G = 1; G <= std::min(nbb, 8); G *= 2) {
+        SweepShape sh;
+        sh.G = G;
+        sh.threads = kThreads;
+        sh.W = sweep_ring(G);
+        sh.smem = sizeof(double) * (size_t)G * sh.W;
+        if (sh.W < 6 * ctx->stream_width) break;
+        const PlanSum rounds = plan_sum(ctx, [G](int w) { return (w * G + kThreads - 1) / kThreads; });
+        const PlanSum steps = plan_sum(ctx, [G](int w) { return (w * G + 31) / 32; });
+        for (int sum = 0; sum < 2; ++sum) {
+            sh.margin = sum != 0;
+            const double c =
+                (sum ? 0.0 : margin) +
+                wave_cost((nbb + G - 1) / G * ctx->n_dir, kFit, sms, [&](bool longest, int share) {
+                    const auto of = [&](const PlanSum& v) { return longest ? v.most : v.mean; };
+                    return std::max(of(rounds) * kc.round * (1 + kc.crowd * (share - 1)),
+                                    of(steps) * share * (kc.fp64 + (sum ? kc.sum : 0.0)));
+                });
+            if (c < best) {
+                best = c;
+                *out = sh;
+            }
+        }
+    }
+    return best;
+}
+
+// The sweep kernel and its shape for batches of nbb bands into ctx->sweep_shape
+// (*found = false: neither model has one).  The stream kernel leaves the margin to
+// the closing reduction, where each direction of a small state costs 250 to 540
+// cycles of latency: k_sweep, whose FP64 pipe is idle then, sums it at no cost.
+// That decides for many directions or bands on few cells (an outer iteration, stream
+// -> level: 800 triangles x 8 bands x 512 directions 461 -> 250 us, 800 x 24 x 128
+// 215 -> 143, 162 x 24 x 32 62 -> 64; tetrahedra x 128 directions, 750 x 20 bands 163 ->
+// 126, 1,296 x 12 163 -> 133, 3,072 x 12 236 -> 234, 750 x 1 58 -> 72).  Over 212 plans
+// the choice costs 0.6 % on average and 15 % at most, the stream kernel always 10 %
+// and 138 %.  k_sweep has to be 4 % and kLevelGain cycles (1 us) faster.
+constexpr double kLevelGain = 2000;
+static bte_status sweep_choose(bte_ctx* ctx, int nbb, bool only_stream, bool* found) {
+    *found = false;
+    int sms = 0, smem_max = 0;
+    BTE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    SweepShape sh;
+    double cost = kNoShape;
+    int annex = ctx->stream_width / 16 + 8;
+    bte_status s = stream_choose(ctx, nbb, annex, &sh, &cost);
+    if (s != BTE_OK || cost == kNoShape) return s;
+    if (!only_stream && ctx->plan_lagged_dirs == 0) {  // (sweeps over lagged edges cannot sum the margin)
+        const int NB = ctx->n_band, batches = (NB + nbb - 1) / nbb;
+        const double warps = (double)bte::reduce_groups(ctx->n) * NB;
+        const double margin =
+            ctx->n_dir * (bte::reduce_by_cells(ctx->n, NB, ctx->n_dir)
+                              ? 23.0 * std::min(NB, 4)
+                              : std::max(250 + 290 * std::min(1.0, warps / 600), 38 * warps / sms));
+        SweepShape level;
+        const double lc = level_choose(ctx, nbb, sms, margin / batches, &level);
+        if (1.04 * lc * batches + kLevelGain < cost * batches + margin) {
+            ctx->sweep_shape = level;
             *found = true;
             return BTE_OK;
         }
-        annex = best.A;  // more than assumed: choose again
     }
-    return BTE_OK;
+    s = stream_plan(ctx);
+    for (int tries = 0; s == BTE_OK && cost < kNoShape && tries < 4; ++tries) {
+        s = stream_annex(ctx, sh);
+        if (s == BTE_OK && sh.smem <= (size_t)smem_max) {
+            ctx->sweep_shape = sh;
+            *found = true;
+            return BTE_OK;
+        }
+        annex = sh.A;  // more than assumed: choose again
+        if (s == BTE_OK) s = stream_choose(ctx, nbb, annex, &sh, &cost);
+    }
+    return s;
 }
 
 // One sweep of bands b0 .. b0+nbb-1 in every direction with shape sh, for the
@@ -2201,11 +2320,11 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
     const int only_shape = sweep_shape_restriction();
     const SweepTuneKey tkey{ctx->device, ctx->n, ctx->F, ctx->n_dir, nbb, ctx->plan_levels, only_margin, only_kernel,
                             only_shape};
-    // the stream kernel, unless the environment asks for another one or this
-    // plan does not suit it
+    // by the models, unless the environment asks for another kernel or shape or
+    // this plan does not suit the stream kernel
     if (!ctx->sweep_tuned && only_margin < 0 && only_shape < 0 && (only_kernel < 0 || only_kernel == 3)) {
         bool found = false;
-        bte_status s2 = stream_choose(ctx, nbb, &found);
+        bte_status s2 = sweep_choose(ctx, nbb, only_kernel == 3, &found);
         if (s2 != BTE_OK) return s2;
         ctx->sweep_tuned = found;
     }
