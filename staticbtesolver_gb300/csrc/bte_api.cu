@@ -1388,6 +1388,17 @@ static bte_status stream_plan(bte_ctx* ctx) {
     return BTE_OK;
 }
 
+// Gives the stream kernel's arrays back; a later plan or attempt starts anew.
+static void stream_release(bte_ctx* ctx) {
+    cudaGetLastError();  // (a failed allocation)
+    for (DevBuf* b : {&ctx->st_lrow, &ctx->st_pos, &ctx->st_cell, &ctx->st_voi, &ctx->st_kinv, &ctx->st_rec, &ctx->st_far,
+                      &ctx->st_nfar})
+        b->release();
+    ctx->stream_lists.clear();
+    ctx->stream_ready = false;
+    ctx->stream_key[0] = 0;
+}
+
 // Launch a kernel, optionally bracketed by profiling events.
 #define BTE_LAUNCH(kind, iter, bytes_fixed, bytes_per_active, ...)                      \
     do {                                                                                \
@@ -2143,56 +2154,6 @@ static double level_choose(bte_ctx* ctx, int nbb, int sms, double margin, SweepS
     return best;
 }
 
-// The sweep kernel and its shape for batches of nbb bands into ctx->sweep_shape
-// (*found = false: neither model has one).  The stream kernel leaves the margin to
-// the closing reduction, where each direction of a small state costs 250 to 540
-// cycles of latency: k_sweep, whose FP64 pipe is idle then, sums it at no cost.
-// That decides for many directions or bands on few cells (an outer iteration, stream
-// -> level: 800 triangles x 8 bands x 512 directions 461 -> 250 us, 800 x 24 x 128
-// 215 -> 143, 162 x 24 x 32 62 -> 64; tetrahedra x 128 directions, 750 x 20 bands 163 ->
-// 126, 1,296 x 12 163 -> 133, 3,072 x 12 236 -> 234, 750 x 1 58 -> 72).  Over 212 plans
-// the choice costs 0.6 % on average and 15 % at most, the stream kernel always 10 %
-// and 138 %.  k_sweep has to be 4 % and kLevelGain cycles (1 us) faster.
-constexpr double kLevelGain = 2000;
-static bte_status sweep_choose(bte_ctx* ctx, int nbb, bool only_stream, bool* found) {
-    *found = false;
-    int sms = 0, smem_max = 0;
-    BTE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    SweepShape sh;
-    double cost = kNoShape;
-    int annex = ctx->stream_width / 16 + 8;
-    bte_status s = stream_choose(ctx, nbb, annex, &sh, &cost);
-    if (s != BTE_OK || cost == kNoShape) return s;
-    if (!only_stream && ctx->plan_lagged_dirs == 0) {  // (sweeps over lagged edges cannot sum the margin)
-        const int NB = ctx->n_band, batches = (NB + nbb - 1) / nbb;
-        const double warps = (double)bte::reduce_groups(ctx->n) * NB;
-        const double margin =
-            ctx->n_dir * (bte::reduce_by_cells(ctx->n, NB, ctx->n_dir)
-                              ? 23.0 * std::min(NB, 4)
-                              : std::max(250 + 290 * std::min(1.0, warps / 600), 38 * warps / sms));
-        SweepShape level;
-        const double lc = level_choose(ctx, nbb, sms, margin / batches, &level);
-        if (1.04 * lc * batches + kLevelGain < cost * batches + margin) {
-            ctx->sweep_shape = level;
-            *found = true;
-            return BTE_OK;
-        }
-    }
-    s = stream_plan(ctx);
-    for (int tries = 0; s == BTE_OK && cost < kNoShape && tries < 4; ++tries) {
-        s = stream_annex(ctx, sh);
-        if (s == BTE_OK && sh.smem <= (size_t)smem_max) {
-            ctx->sweep_shape = sh;
-            *found = true;
-            return BTE_OK;
-        }
-        annex = sh.A;  // more than assumed: choose again
-        if (s == BTE_OK) s = stream_choose(ctx, nbb, annex, &sh, &cost);
-    }
-    return s;
-}
-
 // One sweep of bands b0 .. b0+nbb-1 in every direction with shape sh, for the
 // plan's face slots (2 in 1D and 2D, 3 in 3D).
 template <bool MARGIN>
@@ -2285,6 +2246,62 @@ static bte_status prepare_shape(bte_ctx* ctx, const SweepShape& sh) {
         if (s != BTE_OK) return s;
     }
     return sh.staged ? staged_records(ctx) : BTE_OK;
+}
+
+// The sweep kernel and its shape for batches of nbb bands into ctx->sweep_shape
+// (*found = false: neither model has one).  The stream kernel leaves the margin to
+// the closing reduction, where each direction of a small state costs 250 to 540
+// cycles of latency: k_sweep, whose FP64 pipe is idle then, sums it at no cost.
+// That decides for many directions or bands on few cells (an outer iteration, stream
+// -> level: 800 triangles x 8 bands x 512 directions 461 -> 250 us, 800 x 24 x 128
+// 215 -> 143, 162 x 24 x 32 62 -> 64; tetrahedra x 128 directions, 750 x 20 bands 163 ->
+// 126, 1,296 x 12 163 -> 133, 3,072 x 12 236 -> 234, 750 x 1 58 -> 72).  Over 212 plans
+// the choice costs 0.6 % on average and 15 % at most, the stream kernel always 10 %
+// and 138 %.  k_sweep has to be 4 % and kLevelGain cycles (1 us) faster.
+constexpr double kLevelGain = 2000;
+static bte_status sweep_choose(bte_ctx* ctx, int nbb, bool only_stream, bool* found) {
+    *found = false;
+    int sms = 0, smem_max = 0;
+    BTE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    BTE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    SweepShape sh;
+    double cost = kNoShape;
+    int annex = ctx->stream_width / 16 + 8;
+    bte_status s = stream_choose(ctx, nbb, annex, &sh, &cost);
+    if (s != BTE_OK || cost == kNoShape) return s;
+    if (!only_stream && ctx->plan_lagged_dirs == 0) {  // (sweeps over lagged edges cannot sum the margin)
+        const int NB = ctx->n_band, batches = (NB + nbb - 1) / nbb;
+        const double warps = (double)bte::reduce_groups(ctx->n) * NB;
+        const double margin =
+            ctx->n_dir * (bte::reduce_by_cells(ctx->n, NB, ctx->n_dir)
+                              ? 23.0 * std::min(NB, 4)
+                              : std::max(250 + 290 * std::min(1.0, warps / 600), 38 * warps / sms));
+        SweepShape level;
+        const double lc = level_choose(ctx, nbb, sms, margin / batches, &level);
+        if (1.04 * lc * batches + kLevelGain < cost * batches + margin) {
+            ctx->sweep_shape = level;
+            *found = true;
+            return BTE_OK;
+        }
+    }
+    s = stream_plan(ctx);
+    for (int tries = 0; s == BTE_OK && cost < kNoShape && tries < 4; ++tries) {
+        s = stream_annex(ctx, sh);
+        if (s != BTE_OK) break;
+        if (sh.smem <= (size_t)smem_max) {
+            s = prepare_shape(ctx, sh);
+            if (s != BTE_OK) break;
+            ctx->sweep_shape = sh;
+            *found = true;
+            return BTE_OK;
+        }
+        annex = sh.A;  // more than assumed: choose again
+        s = stream_choose(ctx, nbb, annex, &sh, &cost);
+    }
+    // no annex that fits, or no memory for the padded plan, up to twice what
+    // k_sweep's takes: its arrays make room for k_sweep
+    stream_release(ctx);
+    return s == BTE_ERR_OUT_OF_MEMORY ? BTE_OK : s;
 }
 
 // Solve all systems of one batch by upwind sweeps (exact in one sweep when no
