@@ -51,11 +51,12 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double (*smem)[NWARP])
         }
 }
 
-// a / b for finite a and b with rb = 1 / b rounded, correctly rounded but for
-// over- and underflow (Markstein's theorem: one residual step); 3 operations.
+// a / b with rb = 1 / b rounded, correctly rounded but for underflow (Markstein's
+// theorem: one residual step); 3 operations.  The residual of an infinite a or b, a
+// zero b or a quotient that overflows is not finite, and a rb is the quotient.
 __device__ __forceinline__ double div_by(double a, double b, double rb) {
-    const double q = a * rb;
-    return fma(fma(-q, b, a), rb, q);
+    const double q = a * rb, r = fma(-q, b, a);
+    return (__double2hiint(r) & 0x7ff00000) == 0x7ff00000 ? q : fma(r, rb, q);
 }
 
 // Serial sum of the per-chunk partials (for kernels with one thread per system).
