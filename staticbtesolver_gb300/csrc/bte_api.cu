@@ -3040,11 +3040,12 @@ extern "C" bte_status bte_solve(bte_ctx* ctx, const bte_options* opts, bte_repor
                        ctx->e_curr, ctx->d_bf_cell.as<int>(), ctx->d_hw.as<double>(), ctx->nbf, ND, Np,
                        ctx->d_hpart.as<double>()));
     }
-    if (ctx->n_bc > 0)
+    if (ctx->n_bc > 0) {
         bte::k_heat_final<<<ctx->n_bc, bte::THREADS, 0, st>>>(
             ctx->d_hpart.as<double>(), ctx->d_bf_bc.as<int>(), ctx->d_bf_area.as<double>(), ctx->d_vg.as<double>(),
             ctx->nbf, NB, ctx->dim, ctx->d_qband.as<double>(), ctx->d_q.as<double>());
-    BTE_LAUNCHED();
+        BTE_LAUNCHED();
+    }
     int dsa_stat[4] = {0, 0, 0, 0};
     if (dsa_on && rep.dsa_solves > 0)
         BTE_CUDA(cudaMemcpyAsync(dsa_stat, ctx->cg_stat.p, sizeof(dsa_stat), cudaMemcpyDeviceToHost, st));
