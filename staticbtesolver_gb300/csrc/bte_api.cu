@@ -259,10 +259,13 @@ struct bte_ctx {
     long long launches = 0;
 };
 
+// A failed call leaves its error with the thread, where the next launch check of
+// any context would find it: it is taken from there when it is reported.
 #define BTE_CUDA(call)                                                                    \
     do {                                                                                  \
         cudaError_t _e = (call);                                                          \
         if (_e != cudaSuccess) {                                                          \
+            cudaGetLastError();                                                           \
             ctx->err = std::string(#call) + ": " + cudaGetErrorString(_e);                \
             return _e == cudaErrorMemoryAllocation ? BTE_ERR_OUT_OF_MEMORY : BTE_ERR_CUDA; \
         }                                                                                 \
@@ -369,6 +372,7 @@ bte_status bte_create(bte_ctx** out, int device) {
     int count = 0;
     cudaError_t e = cudaGetDeviceCount(&count);
     if (e != cudaSuccess || count == 0) {
+        cudaGetLastError();
         g_create_error = std::string("no CUDA device: ") + cudaGetErrorString(e);
         return BTE_ERR_NO_DEVICE;
     }
@@ -376,6 +380,7 @@ bte_status bte_create(bte_ctx** out, int device) {
     device %= count;
     e = cudaSetDevice(device);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         g_create_error = cudaGetErrorString(e);
         return BTE_ERR_CUDA;
     }
@@ -385,6 +390,7 @@ bte_status bte_create(bte_ctx** out, int device) {
     if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_pinned, 4 * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_pinned_i, 4 * sizeof(int));
     if (e != cudaSuccess) {
+        cudaGetLastError();
         g_create_error = cudaGetErrorString(e);
         delete ctx;
         return BTE_ERR_CUDA;
@@ -1390,7 +1396,6 @@ static bte_status stream_plan(bte_ctx* ctx) {
 
 // Gives the stream kernel's arrays back; a later plan or attempt starts anew.
 static void stream_release(bte_ctx* ctx) {
-    cudaGetLastError();  // (a failed allocation)
     for (DevBuf* b : {&ctx->st_lrow, &ctx->st_pos, &ctx->st_cell, &ctx->st_voi, &ctx->st_kinv, &ctx->st_rec, &ctx->st_far,
                       &ctx->st_nfar})
         b->release();
@@ -3407,6 +3412,7 @@ static cudaError_t noalloc_scratch_address(double** out) {
     do {                                                                              \
         cudaError_t _e = (call);                                                      \
         if (_e != cudaSuccess) {                                                      \
+            cudaGetLastError();                                                       \
             g_create_error = std::string("bte_bicgstab_csr_noalloc: ") + #call + ": " + \
                              cudaGetErrorString(_e);                                  \
             if (launched) cudaStreamSynchronize(st);                                  \
@@ -3525,6 +3531,7 @@ struct MlpWork {
     do {                                                                                        \
         cudaError_t _e = (call);                                                                \
         if (_e != cudaSuccess) {                                                                \
+            cudaGetLastError();                                                                 \
             g_create_error = std::string("mlp: ") + #call + ": " + cudaGetErrorString(_e);      \
             return _e == cudaErrorMemoryAllocation ? BTE_ERR_OUT_OF_MEMORY : BTE_ERR_CUDA;      \
         }                                                                                       \
