@@ -365,7 +365,7 @@ class Context:
         self._check(_cuda.bte_get_sweep_tuning(self._h, *[c.ctypes.data_as(C.c_void_p) for c in cols], m,
                                                C.byref(n)))
         return [dict(group=int(cols[0][k]), threads=int(cols[1][k]), ring=int(cols[2][k]),
-                     kernel=("level", "staged", "split", "stream")[int(cols[3][k])], ms=float(cols[4][k])) for k in range(m)]
+                     kernel=("level", "staged", "split")[int(cols[3][k])], ms=float(cols[4][k])) for k in range(m)]
 
     def level_order(self, d):
         """The sweep plan's level order of direction d: (cells in order, level starts then n)."""

@@ -120,7 +120,7 @@ struct SweepShape {
     bool staged = false;  // k_sweep_staged (levels staged by bulk copies, right-hand side formed a stage ahead)
     bool split = false;   // k_sweep over the levels split into slices of cap positions (one per thread)
     bool stream = false;  // k_sweep_stream
-    int cap = 0;          // staged, split, stream: positions per stage
+    int cap = 0;          // staged, split: positions per stage; stream: of the widest level
     int WC = 0, H = 0, NCH = 0, A = 0;  // stream: StreamShape
     bte::StreamShape stream_shape() const { return {G, WC, H, W, A, NCH, cap}; }
     int kind() const { return stream ? 3 : staged ? 1 : split ? 2 : 0; }
@@ -200,11 +200,10 @@ struct bte_ctx {
     bool rec_ready = false;
     bool level_ready = false;  // the level-ordered arrays above (the level, split and staged kernels')
     // stream kernel: padded positions (row starts of the levels, cell -> position
-    // and back), k/D and V Omega/D by band and position, stage lists by cap;
-    // records, annex entries and their counts for one (W, cap, NCH, A)
+    // and back), k/D and V Omega/D by band and position; records, annex entries
+    // and their counts for one (W, cap, NCH, A)
     bool stream_ready = false;
     DevBuf st_lrow, st_pos, st_cell, st_voi, st_kinv, st_rec, st_far, st_nfar;
-    std::map<int, std::unique_ptr<StageList>> stream_lists;
     std::vector<int> plan_lrow;  // start rows of the levels, as plan_lvl
     int stream_nq = 0, stream_width = 0;  // chunks of the longest direction; positions of the widest level
     int stream_key[4] = {0, 0, 0, 0};
@@ -1300,7 +1299,6 @@ static bte_status build_sweep_plan(bte_ctx* ctx) {
     ctx->plan_lvl.swap(h_lvl);  // (outlive the uploads)
     ctx->plan_lvl_off.swap(h_off);
     ctx->stage_lists.clear();
-    ctx->stream_lists.clear();
     ctx->rec_ready = ctx->level_ready = ctx->stream_ready = false;
     ctx->stream_key[0] = 0;
     // rows of 32 positions, each level from a row of its own
@@ -1399,7 +1397,6 @@ static void stream_release(bte_ctx* ctx) {
     for (DevBuf* b : {&ctx->st_lrow, &ctx->st_pos, &ctx->st_cell, &ctx->st_voi, &ctx->st_kinv, &ctx->st_rec, &ctx->st_far,
                       &ctx->st_nfar})
         b->release();
-    ctx->stream_lists.clear();
     ctx->stream_ready = false;
     ctx->stream_key[0] = 0;
 }
@@ -2169,9 +2166,8 @@ static void launch_sweep(const bte_ctx* ctx, const SweepShape& sh, int nbb, int 
     const double* kinv = ctx->p_kinv.as<double>();
     const int fm = sweep_slots(ctx);
     if (sh.stream) {  // (leaves the margin to k_reduce)
-        const StageList* sl = ctx->stream_lists.find(sh.cap)->second.get();
         const bte::StreamPlan pl{ctx->st_rec.as<unsigned char>(), ctx->st_far.as<unsigned>(), ctx->st_nfar.as<int>(),
-                                 sl->stages.as<int>(), sl->off.as<int>(), ctx->stream_nq};
+                                 ctx->st_lrow.as<int>(), ctx->p_lvl_off.as<int>(), ctx->stream_nq};
 #define BTE_STREAM_FM(FM)                                                                                            \
     bte::k_sweep_stream<FM><<<grid, sh.threads, sh.smem, st>>>(pl, sh.stream_shape(), ctx->st_kinv.as<double>(),      \
                                                                ctx->st_voi.as<double>(), src, ctx->e_curr,           \
@@ -2214,33 +2210,10 @@ static void launch_sweep(const bte_ctx* ctx, const SweepShape& sh, int nbb, int 
 #undef BTE_SWEEP_FM
 }
 
-// Stage bounds of the stream kernel in rows: the levels, wider ones in slices
-// of at most cap positions.
-static bte_status stream_list(bte_ctx* ctx, int cap) {
-    if (ctx->stream_lists.count(cap)) return BTE_OK;
-    std::vector<int> stages, off(ctx->n_dir + 1, 0);
-    stages.reserve(ctx->plan_lrow.size());
-    for (int d = 0; d < ctx->n_dir; ++d) {
-        off[d] = (int)stages.size();
-        const int l1 = ctx->plan_lvl_off[d + 1] - 1;
-        for (int l = ctx->plan_lvl_off[d]; l < l1; ++l)
-            for (int r = ctx->plan_lrow[l]; r < ctx->plan_lrow[l + 1]; r += cap / 32) stages.push_back(r);
-        stages.push_back(ctx->plan_lrow[l1]);
-    }
-    off[ctx->n_dir] = (int)stages.size();
-    auto sl = std::make_unique<StageList>();
-    BTE_CUDA(upload(sl->stages, stages, ctx->stream));
-    BTE_CUDA(upload(sl->off, off, ctx->stream));
-    BTE_CUDA(cudaStreamSynchronize(ctx->stream));  // the host arrays go out of scope
-    ctx->stream_lists.emplace(cap, std::move(sl));
-    return BTE_OK;
-}
-
 // What a launch of shape sh reads: its plan, stage lists and records.
 static bte_status prepare_shape(bte_ctx* ctx, const SweepShape& sh) {
     if (sh.stream) {
         bte_status s = stream_plan(ctx);
-        if (s == BTE_OK) s = stream_list(ctx, sh.cap);
         return s == BTE_OK ? stream_records(ctx, sh) : s;
     }
     bte_status s = level_plan(ctx);
@@ -2392,7 +2365,7 @@ static bte_status solve_batch_sweep(bte_ctx* ctx, int b0, int nbb, const bte_opt
         // margin only when that saves 3 % of the sweeps and reduction, so a
         // near tie (2D meshes) does not flip between runs.
         bool fuse = false;
-        if (ctx->plan_lagged_dirs == 0 && !ctx->sweep_shape.staged && !ctx->sweep_shape.stream) {  // (the staged kernel leaves it to k_reduce)
+        if (ctx->plan_lagged_dirs == 0 && !ctx->sweep_shape.staged) {  // (the staged kernel leaves it to k_reduce)
             if (only_margin >= 0) fuse = only_margin == 1;
             else {
                 auto time_best = [&](auto&& launch) -> float {

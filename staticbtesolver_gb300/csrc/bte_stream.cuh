@@ -67,7 +67,7 @@ struct StreamShape {
     int G, WC, H; // bands per block, consumer warps per band, helper warps
     int W, A;     // ring positions (a power of two), annex places per chunk
     int NCH;      // chunk buffers (a power of two)
-    int cap;      // positions per stage at most: a level, or a slice of a wider one
+    int cap;      // positions of the widest level
 };
 __host__ __device__ constexpr int stream_ring(int W, int A, int NCH) { return W + 2 + NCH * ((A + 1) / 2 * 2); }
 // Bytes per position of the buffers: its record, and per band k/D and V Omega/D.
@@ -80,11 +80,11 @@ __host__ __device__ constexpr size_t stream_smem_bytes(const StreamShape& s) {
            (size_t)s.NCH * SCH * stream_position_bytes<FM>(s.G);
 }
 // Positions at most `near` back (near = W - cap) are still in the ring
-// throughout the stage that reads them; older ones come from the annex.  They
+// throughout the level that reads them; older ones come from the annex.  They
 // have been written when the helpers fetch them, NCH chunks ahead of their use
 // at most, if W >= cap + (NCH + 1) SCH.  A consumer loads a row of 32 positions
 // before it releases the chunk of its row before, at most 2 WC x 32 - 32
-// positions apart (rows of one stage, or the last of one and the first of the
+// positions apart (rows of one level, or the last of one and the first of the
 // next): both must fit in the NCH buffers.  A barrier's parity tells
 // two successive phases apart only, so whoever waits for a chunk must have seen
 // the chunk before it in the same buffer: a helper has if H divides NCH.
@@ -233,8 +233,8 @@ struct StreamPlan {
     const unsigned char* rec;  // [n_dir][npad]
     const unsigned* far;       // [n_dir][nq][FM SCH]
     const int* nfar;           // [n_dir][nq]
-    const int* stages;         // per direction: start rows of its stages, then its rows
-    const int* stage_off;      // [n_dir + 1]
+    const int* lrow;           // per direction: start rows of its levels, then its rows
+    const int* lvl_off;        // [n_dir + 1]
     int nq;                    // chunks of the longest direction: npad = nq SCH
 };
 
@@ -295,9 +295,9 @@ __global__ void __launch_bounds__(STHREADS, 1) k_sweep_stream(StreamPlan sp, Str
     const int gn = min(sh.G, nbb - g0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t npad = (size_t)sp.nq * SCH;
-    const int* stg = sp.stages + sp.stage_off[d];
-    const int ns = sp.stage_off[d + 1] - sp.stage_off[d] - 1;
-    const int rows = stg[ns], nq = (rows + SCH / 32 - 1) / (SCH / 32);
+    const int* lv = sp.lrow + sp.lvl_off[d];
+    const int ns = sp.lvl_off[d + 1] - sp.lvl_off[d] - 1;
+    const int rows = lv[ns], nq = (rows + SCH / 32 - 1) / (SCH / 32);
     const int qmask = sh.NCH - 1, qshift = __ffs(sh.NCH) - 1;
     if (threadIdx.x == 0) {
         *dead = 0;
@@ -492,28 +492,28 @@ __global__ void __launch_bounds__(STHREADS, 1) k_sweep_stream(StreamPlan sp, Str
         it.kinv = kd[p];
         it.rhs = kd[span + p];
     };
-    // stage bounds: 32 of them in the warp's registers, the next 32 loaded ahead
-    int base = 0, sb = stg[min(lane, ns)], sbn = stg[min(32 + lane, ns)];
+    // level bounds: 32 of them in the warp's registers, the next 32 loaded ahead
+    int base = 0, sb = lv[min(lane, ns)], sbn = lv[min(32 + lane, ns)];
     auto bound = [&](int i) {  // i never goes back, nor ahead by more than 1
         if (i - base == 32) {
             base += 32;
             sb = sbn;
-            sbn = stg[min(base + 32 + lane, ns)];
+            sbn = lv[min(base + 32 + lane, ns)];
         }
         return __shfl_sync(0xffffffffu, sb, i - base);
     };
-    // Row by row through a stage (rows wl, wl + WC, ... of it), then on to the
-    // next stage behind the band's barrier.  The row after the current one is
+    // Row by row through a level (rows wl, wl + WC, ... of it), then on to the
+    // next level behind the band's barrier.  The row after the current one is
     // loaded before the current one is solved, so a barrier is followed by the
     // loads of upstream values and the FP64 chain only.
     int s = 0;
     int r = wl, rB = bound(min(1, ns)), rC = bound(min(2, ns)), rD = bound(min(3, ns));
     bool has = ns > 0 && r < rB;
     auto step = [&](Item& cur, Item& nxt) {
-        const bool last = r + WC >= rB;  // of this stage, for this warp
+        const bool last = r + WC >= rB;  // of this level, for this warp
         const int rn = last ? rB + wl : r + WC, re = last ? rC : rB;
         const bool more = rn < re;
-        // (a warp without a row in the next stage sees this stage's to their end)
+        // (a warp without a row in the next level sees this level's to their end)
         const int upto = more ? rn : rB, seen = more ? rn : rB - 1;
         if (seen >= known) need(seen);
         if (more) load(rn, nxt);
@@ -534,13 +534,13 @@ __global__ void __launch_bounds__(STHREADS, 1) k_sweep_stream(StreamPlan sp, Str
             ++s;
             rB = rC;
             rC = rD;
-            rD = bound(min(s + 3, ns));  // (used a stage later)
+            rD = bound(min(s + 3, ns));  // (used a level later)
         }
         has = more && ok;  // (after a failed wait nothing is solved any more)
         r = rn;
     };
     Item A, B;
-    if (ns > 0) {  // the first row, or the first stage's end
+    if (ns > 0) {  // the first row, or the first level's end
         need(min(r, rB - 1));
         if (has) load(r, A);
         release(min(r, rB));
