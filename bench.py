@@ -187,14 +187,18 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-def ncu_traffic(kernel, workload):
+SWEEP_KERNELS = ("k_sweep", "k_sweep_staged", "k_sweep (split)", "k_sweep_stream")  # bte_report.sweep_kernel
+
+
+def ncu_traffic(kernel, workload, ran=None):
     """DRAM bytes per launch of `kernel` on `workload` from the committed ncu summaries, if any
-    (a table row "| kernel | ... | traffic_bytes_per_launch=X |" in profiles/*<workload>*.md)."""
+    (a table row "| kernel | ... | traffic_bytes_per_launch=X |" in profiles/*<workload>*.md); with `ran`,
+    the name of the function that was launched, only from a row that names it."""
     for path in sorted(glob.glob(os.path.join(ROOT, "profiles", f"*{workload}*.md"))):
         for line in open(path):
             m = re.match(r"\|\s*" + re.escape(kernel) + r"\s*\|.*\|\s*traffic_bytes_per_launch=([0-9.eE+]+)\s*\|",
                          line)
-            if m:
+            if m and (ran is None or re.search(r"\b" + re.escape(ran) + r"\b", line)):
                 return float(m.group(1)), os.path.relpath(path, ROOT)
     return None, None
 
@@ -470,12 +474,14 @@ def run_ours(args, rank, world, local):
         tot_ms = sum(v["ms"] for v in stats.values())
         peak, peak_kind = measured_peaks()
         achieved = dom["bytes"] / (dom["ms"] / 1e3) / 1e9
-        traffic, traffic_src = ncu_traffic(dom_name, args.workload)
+        sweep_fn = SWEEP_KERNELS[last["sweep_kernel"]]
+        traffic, traffic_src = ncu_traffic(dom_name, args.workload,
+                                           sweep_fn.split()[0] if dom_name == "upwind_sweep" else None)
         sweep = stats.get("upwind_sweep", {})
         sweep_roof = None
         if sweep.get("launches") and dom_name != "upwind_sweep":
             s_ach = sweep["bytes"] / (sweep["ms"] / 1e3) / 1e9
-            s_tr, s_tr_src = ncu_traffic("upwind_sweep", args.workload)
+            s_tr, s_tr_src = ncu_traffic("upwind_sweep", args.workload, sweep_fn.split()[0])
             sweep_roof = {"bound": "hbm", "kernel": "upwind_sweep", "achieved": round(s_ach, 1), "peak": peak,
                           "unit": "GB/s", "frac": round(s_ach / peak, 4), "traffic": s_tr, "traffic_source": s_tr_src,
                           "algorithmic_bytes_per_launch": sweep["bytes"] / sweep["launches"],
@@ -521,8 +527,7 @@ def run_ours(args, rank, world, local):
                        "mixed_fp32_fp64_form": mixed,
                        "sweep_shape": {"bands_per_block": last["sweep_group"], "threads": last["sweep_threads"],
                                        "ring": last["sweep_ring"],
-                                       "kernel": ("k_sweep", "k_sweep_staged", "k_sweep (split)",
-                                                  "k_sweep_stream")[last["sweep_kernel"]],
+                                       "kernel": sweep_fn,
                                        "margin_summed_in": "sweep" if last["sweep_margin"] else "k_reduce"},
                        "speedup_vs_plain_fp64": (plain["s_extrapolated"] / t_step)
                        if plain and "s_extrapolated" in plain else None},
@@ -534,8 +539,8 @@ def run_ours(args, rank, world, local):
                          "note": ("the low-order solve (k_dsa_pcg and its small helpers): L2-resident, bound by one "
                                   "grid barrier per conjugate-gradient iteration; bytes = iterations x cells x "
                                   "algorithmic bytes per cell and iteration" if dom_name == "dsa_correction" else
-                                  "dependency chain of the level-ordered substitution (barrier per level, FP64 "
-                                  "chain per item)" if dom_name == "upwind_sweep" else None)},
+                                  "dependency chain of the level-ordered substitution and the FP64 pipe"
+                                  if dom_name == "upwind_sweep" else None)},
             "roofline_sweep": sweep_roof,
             "cpu_baseline": cpu,
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
