@@ -74,7 +74,9 @@ typedef struct bte_options {
     bte_iteration_cb on_iteration; /* may be NULL */
     void* user;
     int profile;          /* nonzero: time every inner-solve kernel with CUDA events
-                             (bte_get_kernel_stats); adds event records between launches */
+                             (bte_get_kernel_stats); adds event records between launches.  PLAIN and
+                             MIXED then take one launch per phase also where an ordinary solve has
+                             one launch per batch (BTE_KRYLOV): other last bits, and longer */
     int accel;            /* outer-iteration acceleration: 0 none (the reference), 1 learned
                              (the MLP set by bte_set_mlp), 2 Aitken per cell (non-learned),
                              3 Anderson mixing of T and the boundary-cell intensities

@@ -1464,9 +1464,10 @@ static cudaLaunchConfig_t cluster_config(int S, int ctas, int len, int slots, bo
 // Cells per CTA for S systems of n cells, or 0: the phase kernels (more than
 // KC_CTAS CTAs' cells, or clusters that do not fit the device).  A system gets
 // the fewest CTAs its cells need: remote neighbour values and cluster barriers
-// cost more than a fuller SM (20,000 cells x 256 systems: 10 CTAs 81 ms, 12
-// 107 ms, 16 172 ms; 10,082 cells in FP32: 5 CTAs 25 ms, 6 28 ms, 8 38 ms).
-// While that leaves SMs without one it gets more, of at least kClusterSpread
+// cost more than a fuller SM (two outer iterations of 256 systems: 4,050 triangles
+// in FP64 with 2 CTAs 8.7 ms, 4 9.1, 6 10.9, 8 13.0; 2,048 with 1 4.1, 4 4.9, 8 7.1;
+// 3,072 tetrahedra with 2 3.0, 4 3.5, 8 5.1; 10,082 triangles in FP32 with 5 17.0,
+// 6 19.4, 8 25.5).  While that leaves SMs without one it gets more, of at least kClusterSpread
 // cells (578 cells x 32 systems: 1 CTA and 4 CTAs 17 ms, the barriers then cost
 // what the FP64 pipes gain).
 constexpr int kClusterSpread = 512;
@@ -1557,8 +1558,8 @@ static bte_status batch_len(bte_ctx* ctx, int S, int prec, int* len) {
 }
 
 // One CSR system whose rows have at most `most` entries: slots (0: the phase
-// kernels, for longer rows, more unknowns than a cluster holds, and under
-// BTE_KRYLOV=phase) and cells per CTA.  The other SMs are idle, so a system gets
+// kernels, for longer rows, more unknowns than a cluster holds -- 32,768, with five
+// to eight entries a row 28,672 -- and under BTE_KRYLOV=phase) and cells per CTA.  The other SMs are idle, so a system gets
 // a CTA for every 256 unknowns, up to a cluster's 16 (2,048 unknowns, 82 steps:
 // of 64, 128, 256, 512 and 1,024 each 775, 772, 745, 815, 965 us; 3,872: 1,048,
 // 1,059, 1,100, 1,136, 1,449 us).

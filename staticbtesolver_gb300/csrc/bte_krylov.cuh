@@ -34,7 +34,9 @@
 // loads), 32,768 unknowns 20.5 -> 5.6 ms.
 // Sums are taken in a fixed order (threads, warps, CTAs), so a solve is
 // reproducible to the bit; they are grouped differently from the phase
-// kernels', so the two agree to rounding.
+// kernels', so the two agree to rounding.  The FP64 pipe of the SMs with a CTA is
+// 50 % busy on 578 triangles, 54 % on 750 tetrahedra, 43 % in FP32 on 10,082
+// triangles (the scalars and sums); barriers and shared-memory latency are the rest.
 #pragma once
 #include "bte_kernels.cuh"
 

@@ -33,11 +33,12 @@
 // Per cell the arithmetic is k_sweep's in its order, so x is the same to the
 // bit.
 //
-// Measured, one launch in ms, k_sweep with the shape it was timed into -> here:
-// square 1,024 x 5 bands 0.068 -> 0.038, 20,000 x 40 0.588 -> 0.378, 25,088 x 20
-// 0.545 -> 0.290, 100,352 x 20 1.71 -> 1.00; cube 48,000 x 7 1.28 -> 0.84,
-// 131,712 x 20 8.9 -> 6.32.  Now the FP64 pipe is 65 % busy at the large sizes;
-// a narrow level costs ~500 cycles of control and latency per row.
+// Measured, one launch in ms by events around it, k_sweep with the shape it is timed
+// into -> here: triangles, 1,058 x 5 bands 0.055 -> 0.039, 20,000 x 40 0.529 -> 0.407,
+// 25,088 x 20 0.509 -> 0.309, 100,352 x 20 1.50 -> 1.07; tetrahedra, 48,000 x 7
+// 1.23 -> 0.89, 131,712 x 20 8.95 -> 6.53.  The FP64 pipe of the SMs with a block is
+// 60 to 73 % busy at the large sizes (70 on 100,352 x 20, 73 on 20,000 x 40, 60 on
+// 48,000 x 7); a narrow level costs ~500 cycles of control and latency per row.
 // Without gain: two bands per consumer warp, unpadded rows, every helper on
 // every chunk.
 #pragma once
