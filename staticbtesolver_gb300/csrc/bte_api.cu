@@ -2045,10 +2045,10 @@ static double wave_cost(int blocks, int fit, int sms, F&& block) {
 //    sides, NCH chunks in flight;
 //  * on tetrahedra, the bytes of records and coefficients.
 // The constants (cycles) were fitted to ~90 shapes on each of 189 plans (162 to
-// 39,200 triangles x 1 to 40 bands, 162 to 55,566 tetrahedra x 1 to 20 bands): the
-// shape picked takes 1.1 % (2D) and 1.4 % (3D) longer than the fastest on average, 8 %
-// and 15 % at most; on 18 other plans, up to 100,352 triangles and 131,712 tetrahedra,
-// 1 % and 8 %.  (With the mean rows per level in place of the turns and no helpers' time
+// 39,200 triangles x 1 to 40 bands, 162 to 55,566 tetrahedra x 1 to 20 bands).  With 109
+// more of other sizes and bands the shape picked takes 1.1 % (2D) and 1.7 % (3D) longer
+// than the fastest on average, 8 % and 15 % at most; on 18 plans of up to 100,352
+// triangles and 131,712 tetrahedra 1 % and 8 %.  (With the mean rows per level in place of the turns and no helpers' time
 // per band it picked shapes up to 80 % longer: 16,464 tetrahedra x 16 bands 1,126 us,
 // now 666; 2,450 triangles x 24 bands 113 us, now 63.)  A plan of a new mesh costs no
 // trial sweeps (~20, 100 ms on 100,352 triangles).
